@@ -27,7 +27,8 @@ torch::Tensor spfa_coo_cuda_forward(torch::Tensor Q, torch::Tensor K, torch::Ten
     TORCH_CHECK(W_row_ind.dim() == 1 && W_col_ind.dim() == 1 && W_row_ind.size(0) == W_col_ind.size(0),
                 "W_row_ind and W_col_ind must be 1-D with one entry per mask non-zero");
     c10::cuda::CUDAGuard guard(Q.device());
-    Workspace ws(spfa_coo_min_workspace_bytes(Q.size(0)), Q.device());
+    Workspace ws(spfa_coo_min_workspace_bytes(Q.size(0)) +
+                     spfa_csr_workspace_bytes_16(Q.size(0), W_row_ind.size(0), (int)Q.size(1)), Q.device());
     raise_for_status(spfa_coo_forward_16(dtype_code(Q), Q.data_ptr(), K.data_ptr(), V.data_ptr(),
                                          u64_ptr(W_row_ind, "W_row_ind"), u32_ptr(W_col_ind, "W_col_ind"), W_row_ind.size(0),
                                          m.data_ptr(), l.data_ptr(), O.data_ptr(), /*row_begin=*/0, Q.size(0), K.size(0),

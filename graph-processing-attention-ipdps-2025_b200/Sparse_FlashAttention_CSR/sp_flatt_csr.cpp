@@ -27,10 +27,11 @@ torch::Tensor spfa_csr_cuda_forward(torch::Tensor Q, torch::Tensor K, torch::Ten
     TORCH_CHECK(W_row_off.dim() == 1 && W_row_off.size(0) == Q.size(0) + 1, "W_row_off must have L+1 entries");
     TORCH_CHECK(W_col_ind.dim() == 1, "W_col_ind must be 1-D");
     c10::cuda::CUDAGuard guard(Q.device());
-    raise_for_status(spfa_csr_forward_16(dtype_code(Q), Q.data_ptr(), K.data_ptr(), V.data_ptr(),
-                                         u64_ptr(W_row_off, "W_row_off"), u32_ptr(W_col_ind, "W_col_ind"), W_col_ind.size(0),
-                                         m.data_ptr(), l.data_ptr(), O.data_ptr(), Q.size(0), K.size(0), (int)Q.size(1),
-                                         use_nan ? 1 : 0, at::cuda::getCurrentCUDAStream().stream()));
+    Workspace ws(spfa_csr_workspace_bytes_16(Q.size(0), W_col_ind.size(0), (int)Q.size(1)), Q.device());
+    raise_for_status(spfa_csr_forward_16_ws(dtype_code(Q), Q.data_ptr(), K.data_ptr(), V.data_ptr(),
+                                            u64_ptr(W_row_off, "W_row_off"), u32_ptr(W_col_ind, "W_col_ind"), W_col_ind.size(0),
+                                            m.data_ptr(), l.data_ptr(), O.data_ptr(), Q.size(0), K.size(0), (int)Q.size(1),
+                                            use_nan ? 1 : 0, ws.ptr, ws.bytes, at::cuda::getCurrentCUDAStream().stream()));
     return O;
   }
   if (needs_float32_copy(Q)) {

@@ -37,7 +37,7 @@ EXPORTS = (
     "spfa_dense_mask_offsets", "spfa_dense_mask_fill", "spfa_bigbird_workspace_bytes", "spfa_bigbird_forward_f32",
     "spfa_local_forward_batched_f32", "spfa_local_1d_dilated_forward_batched_f32", "spfa_local_2d_dilated_forward_batched_f32",
     "spfa_global_no_local_forward_batched_f32", "spfa_csr_forward_batched_f32", "spfa_coo_forward_batched_f32",
-    "spfa_csr_forward_16", "spfa_coo_forward_16", "spfa_local_forward_16", "spfa_local_1d_dilated_forward_16",
+    "spfa_csr_forward_16", "spfa_csr_forward_16_ws", "spfa_csr_workspace_bytes_16", "spfa_coo_forward_16", "spfa_local_forward_16", "spfa_local_1d_dilated_forward_16",
     "spfa_local_2d_dilated_forward_16", "spfa_global_no_local_workspace_bytes_16", "spfa_global_no_local_forward_16",
     "spfa_csr_workspace_bytes_idx32", "spfa_csr_forward_f32_idx32", "spfa_coo_forward_f32_idx32", "spfa_coo_plan_build_idx32",
 )
@@ -90,6 +90,10 @@ def lib() -> ctypes.CDLL:
     L.spfa_coo_plan_build_idx32.argtypes = [vp, vp, i64, i64, i64, i64, i32, vp, sz, vp]
     L.spfa_csr_forward_16.restype = i32
     L.spfa_csr_forward_16.argtypes = [i32] + [vp] * 5 + [i64] + [vp] * 3 + [i64, i64, i32, i32, vp]
+    L.spfa_csr_workspace_bytes_16.restype = sz
+    L.spfa_csr_workspace_bytes_16.argtypes = [i64, i64, i32]
+    L.spfa_csr_forward_16_ws.restype = i32
+    L.spfa_csr_forward_16_ws.argtypes = [i32] + [vp] * 5 + [i64] + [vp] * 3 + [i64, i64, i32, i32, vp, sz, vp]
     L.spfa_coo_forward_16.restype = i32
     L.spfa_coo_forward_16.argtypes = [i32] + [vp] * 5 + [i64] + [vp] * 3 + [i64, i64, i64, i32, i32, vp, sz, vp]
     L.spfa_local_forward_16.restype = i32
@@ -469,10 +473,12 @@ def forward_16(kind, Q, K, V, m, l, O, *, p0=0, p1=0, global_inds=None, row_off=
         st = _stream(dev)
         q, k, v, mm, ll, oo = (_ptr(t) for t in (Q, K, V, m, l, O))
         if kind == "csr":
-            rc = lib().spfa_csr_forward_16(code, q, k, v, _ptr(_as_u64(row_off)), _ptr(_as_u32(col_ind)), col_ind.shape[0],
-                                           mm, ll, oo, n_rows, Lk, d, int(use_nan), st)
+            buf, wp, wb = workspace(lib().spfa_csr_workspace_bytes_16(n_rows, col_ind.shape[0], d), dev)
+            rc = lib().spfa_csr_forward_16_ws(code, q, k, v, _ptr(_as_u64(row_off)), _ptr(_as_u32(col_ind)), col_ind.shape[0],
+                                              mm, ll, oo, n_rows, Lk, d, int(use_nan), wp, wb, st)
         elif kind == "coo":
-            buf, wp, wb = workspace(lib().spfa_coo_min_workspace_bytes(n_rows), dev)
+            buf, wp, wb = workspace(lib().spfa_coo_min_workspace_bytes(n_rows) +
+                                    lib().spfa_csr_workspace_bytes_16(n_rows, col_ind.shape[0], d), dev)
             rc = lib().spfa_coo_forward_16(code, q, k, v, _ptr(_as_u64(row_ind)), _ptr(_as_u32(col_ind)), col_ind.shape[0],
                                            mm, ll, oo, row_begin, n_rows, Lk, d, int(use_nan), wp, wb, st)
         else:

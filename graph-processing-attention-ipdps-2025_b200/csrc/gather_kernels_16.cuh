@@ -54,11 +54,21 @@ __device__ __forceinline__ Vec8 ldg8(const T* p) {  // 16 bytes = 8 elements, re
   return r;
 }
 
-__device__ __forceinline__ float dot8(const Vec8& q, const Vec8& k) {
-  float p = q.v[0] * k.v[0];
-#pragma unroll
-  for (int i = 1; i < 8; ++i) p = fmaf(q.v[i], k.v[i], p);
-  return p;
+// q . k of one 16-byte piece; k stays packed until it is used (eight pieces in flight are 32 registers, not 64).
+template <class T>
+__device__ __forceinline__ float dot8(const Vec8& q, const uint4 k) {
+  float2 f = Cvt16<T>::up(k.x);
+  float p = q.v[0] * f.x;
+  p = fmaf(q.v[1], f.y, p);
+  f = Cvt16<T>::up(k.y);
+  p = fmaf(q.v[2], f.x, p);
+  p = fmaf(q.v[3], f.y, p);
+  f = Cvt16<T>::up(k.z);
+  p = fmaf(q.v[4], f.x, p);
+  p = fmaf(q.v[5], f.y, p);
+  f = Cvt16<T>::up(k.w);
+  p = fmaf(q.v[6], f.x, p);
+  return fmaf(q.v[7], f.y, p);
 }
 
 struct RowAcc8 {
@@ -72,8 +82,8 @@ struct RowAcc8 {
   }
 };
 
-template <int LPK>
-__device__ __forceinline__ void softmax_step4_16(float mine, int grp, const Vec8 (&v)[4], RowAcc8& st) {
+template <int LPK, class T>
+__device__ __forceinline__ void softmax_step4_16(float mine, int grp, const uint4 (&v)[4], RowAcc8& st) {
   float mc = fmaxf(mine, __shfl_xor_sync(kFullMask, mine, LPK / 2));
   mc = fmaxf(mc, __shfl_xor_sync(kFullMask, mc, LPK / 4));
   const float m_new = fmaxf(st.m, mc);
@@ -86,13 +96,17 @@ __device__ __forceinline__ void softmax_step4_16(float mine, int grp, const Vec8
   const float p2 = __shfl_sync(kFullMask, pm, base + LPK / 2);
   const float p3 = __shfl_sync(kFullMask, pm, base + LPK / 2 + LPK / 4);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    float a = st.acc.v[i] * corr;
-    a = fmaf(p0, v[0].v[i], a);
-    a = fmaf(p1, v[1].v[i], a);
-    a = fmaf(p2, v[2].v[i], a);
-    a = fmaf(p3, v[3].v[i], a);
-    st.acc.v[i] = a;
+  for (int i = 0; i < 8; ++i) st.acc.v[i] *= corr;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const float p = (u == 0) ? p0 : (u == 1) ? p1 : (u == 2) ? p2 : p3;
+    const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = Cvt16<T>::up(w[i]);
+      st.acc.v[2 * i] = fmaf(p, f.x, st.acc.v[2 * i]);
+      st.acc.v[2 * i + 1] = fmaf(p, f.y, st.acc.v[2 * i + 1]);
+    }
   }
   st.l = fmaf(st.l, corr, (p0 + p1) + (p2 + p3));
   st.m = m_new;
@@ -109,30 +123,45 @@ __device__ __forceinline__ void accumulate_slots16(const Cols& cols, const typen
   const int own = (((sub & (LPK / 2)) != 0) ? 2 : 0) + (((sub & (LPK / 4)) != 0) ? 1 : 0);
   const T* Kl = K + sub * 8;
   const T* Vl = V + sub * 8;
+  int32_t c_next = (t0 + lane < t1) ? cols.slot(row, t0 + lane) : -1;
   for (int64_t base = t0; base < t1; base += 32) {
-    const int64_t tl = base + lane;
-    const int32_t c_lane = (tl < t1) ? cols.slot(row, tl) : -1;
+    const int32_t c_lane = c_next;  // the next batch's columns travel while this batch's K/V rows are worked on
+    c_next = (base + 32 + lane < t1) ? cols.slot(row, base + 32 + lane) : -1;
+    if (__all_sync(kFullMask, c_lane >= 0)) {  // 32 real keys: no predicates
+#pragma unroll 1
+      for (int j0 = 0; j0 < LPK; j0 += 4) {
+        uint4 k[4], v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const uint32_t c = (uint32_t)__shfl_sync(kFullMask, c_lane, grp + (j0 + u) * KPS);
+          k[u] = __ldg(reinterpret_cast<const uint4*>(Kl + (size_t)c * D));
+          v[u] = __ldg(reinterpret_cast<const uint4*>(Vl + (size_t)c * D));
+        }
+        const float mine = reduce4_transposed<LPK>(dot8<T>(q, k[0]), dot8<T>(q, k[1]), dot8<T>(q, k[2]), dot8<T>(q, k[3]), sub) * scale;
+        softmax_step4_16<LPK, T>(mine, grp, v, st);
+      }
+      continue;
+    }
     const int nb = (t1 - base < 32) ? (int)(t1 - base) : 32;
 #pragma unroll 1
     for (int j0 = 0; j0 < LPK; j0 += 4) {
       if (j0 * KPS >= nb) break;  // warp-uniform
-      Vec8 k[4], v[4];
+      uint4 k[4], v[4];
       int32_t c_own = -1;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int32_t c = __shfl_sync(kFullMask, c_lane, grp + (j0 + u) * KPS);
         if (c >= 0) {
-          k[u] = ldg8<T>(Kl + (size_t)c * D);
-          v[u] = ldg8<T>(Vl + (size_t)c * D);
+          k[u] = __ldg(reinterpret_cast<const uint4*>(Kl + (size_t)c * D));
+          v[u] = __ldg(reinterpret_cast<const uint4*>(Vl + (size_t)c * D));
         } else {  // a masked key contributes probability 0; zero V keeps 0 * V finite
-#pragma unroll
-          for (int i = 0; i < 8; ++i) k[u].v[i] = v[u].v[i] = 0.f;
+          k[u] = v[u] = make_uint4(0u, 0u, 0u, 0u);
         }
         if (u == own) c_own = c;
       }
-      float mine = reduce4_transposed<LPK>(dot8(q, k[0]), dot8(q, k[1]), dot8(q, k[2]), dot8(q, k[3]), sub) * scale;
+      float mine = reduce4_transposed<LPK>(dot8<T>(q, k[0]), dot8<T>(q, k[1]), dot8<T>(q, k[2]), dot8<T>(q, k[3]), sub) * scale;
       if (c_own < 0) mine = neg_inf();
-      softmax_step4_16<LPK>(mine, grp, v, st);
+      softmax_step4_16<LPK, T>(mine, grp, v, st);
     }
   }
 }
@@ -184,29 +213,129 @@ __device__ __forceinline__ void store_row16(const RowAcc8& st, T* __restrict__ m
   }
 }
 
-template <int D, class T, class Cols>
+// Rows cut into slices (explicit masks whose caller gave scratch): a power-law graph holds most of its entries in a few rows,
+// and a row walked by one warp or one CTA is a chain of dependent loads (about a microsecond per 16 keys): at L = 50021,
+// d = 64, 1.96M f16 entries in rows of up to 8192 the launch took 314 us with single-CTA long rows, 300 us when clusters of
+// eight CTAs shared them, because every resident warp that waits for a long row is a load that is not in flight. So rows of
+// more than kSliceSlots slots are cut into slices that single warps walk independently; partial states go to scratch and the
+// warp that finishes a row's last slice folds them in slice order: 109 us for the whole call. A slice is a multiple of the
+// 32-slot batch, long enough that the few partial states cost nothing beside the K/V rows (2 * D * 2 bytes per entry).
+constexpr int kSliceSlots = 256;
+
+struct RowSlices {
+  unsigned int* count;  // slices listed; zero before row_slices_kernel
+  int4* items;          // {row, slice, slices of the row, index of the row's first item}
+  unsigned int* done;   // at a row's first item: slices finished
+  float* part;          // [cap][d + 4]: un-normalised accumulator, then m, l
+  unsigned int cap;
+};
+
+static __global__ void row_slices_kernel(const uint64_t* __restrict__ row_off, int64_t n_rows, const RowSlices sl) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= n_rows) return;
+  const int64_t n = (int64_t)row_off[r + 1] - (int64_t)row_off[r];
+  if (n <= kSliceSlots) return;
+  const unsigned int ns = (unsigned int)((n + kSliceSlots - 1) / kSliceSlots);
+  const unsigned int first = atomicAdd(sl.count, ns);
+  if (first >= sl.cap || ns > sl.cap - first) return;  // not reached with ascending offsets: cap covers 2 nnz / kSliceSlots
+  sl.done[first] = 0u;
+  for (unsigned int s = 0; s < ns; ++s) sl.items[first + s] = make_int4((int)r, (int)s, (int)ns, (int)first);
+}
+
+// One warp per query row at a time, rows claimed from the CTA's counter. With SLICED, blocks [list_begin, list_begin +
+// list_blocks) walk the listed slices, one per warp, and the other blocks leave the listed rows out; the list is produced by
+// the launch before this one, which this one may overlap (only the list blocks wait for it). The list blocks come after a
+// first wave of ordinary blocks, which covers the time the list takes. Without SLICED (implicit masks, or a CSR call without
+// scratch) rows beyond kHeavyRowSlots are shared by the four warps of their CTA.
+template <int D, class T, class Cols, bool SLICED>
 __global__ void __launch_bounds__(kRowWarps * 32, 6)
 gather_rows16_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __restrict__ V, T* __restrict__ m,
                      T* __restrict__ l, T* __restrict__ O, const Cols cols, int64_t row_begin, int64_t n_rows, int use_nan,
-                     float scale) {
+                     float scale, int rows_per_cta, const RowSlices sl, int list_begin, int list_blocks) {
   constexpr int LPK = D / 8;
-  __shared__ int s_heavy[kRowWarps];
-  __shared__ int s_n_heavy;
+  __shared__ int s_heavy[kMaxRowsPerCta];
+  __shared__ int s_n_heavy, s_next;
   __shared__ float s_ml[kRowWarps][2];
   __shared__ float s_acc[kRowWarps][D];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) s_n_heavy = 0;
+  int64_t block = blockIdx.x;
+  if (SLICED) {
+    if ((int)blockIdx.x >= list_begin && (int)blockIdx.x < list_begin + list_blocks) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      const unsigned int n_items = min(*(volatile unsigned int*)sl.count, sl.cap);
+      for (unsigned int it = ((int)blockIdx.x - list_begin) * kRowWarps + warp; it < n_items;
+           it += (unsigned int)list_blocks * kRowWarps) {
+        const int4 item = sl.items[it];
+        const int64_t r = item.x;
+        const typename Cols::Row row = cols.open(r, row_begin + r);
+        const int64_t t0 = (int64_t)item.y * kSliceSlots;
+        const int64_t t1 = (t0 + kSliceSlots < row.n) ? (t0 + kSliceSlots) : row.n;
+        const Vec8 q = ldg8<T>(Q + (size_t)r * D + (lane % LPK) * 8);
+        RowAcc8 st;
+        st.clear();
+        accumulate_slots16<D, T, Cols>(cols, row, t0, t1, q, K, V, scale, lane, st);
+        merge_groups16<LPK>(st);
+        float* part = sl.part + (size_t)it * (D + 4);
+        if (lane < LPK) {
+          float4* a = reinterpret_cast<float4*>(part + lane * 8);
+          a[0] = make_float4(st.acc.v[0], st.acc.v[1], st.acc.v[2], st.acc.v[3]);
+          a[1] = make_float4(st.acc.v[4], st.acc.v[5], st.acc.v[6], st.acc.v[7]);
+        }
+        if (lane == 0) *reinterpret_cast<float2*>(part + D) = make_float2(st.m, st.l);
+        __threadfence();
+        __syncwarp();
+        unsigned int before = 0;
+        if (lane == 0) before = atomicAdd(sl.done + item.w, 1u);
+        if (__shfl_sync(kFullMask, before, 0) != (unsigned int)item.z - 1u) continue;
+        __threadfence();
+        const float* p0 = sl.part + (size_t)item.w * (D + 4);
+        float mx = neg_inf();
+        for (int s = lane; s < item.z; s += 32) mx = fmaxf(mx, __ldcg(p0 + (size_t)s * (D + 4) + D));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(kFullMask, mx, o));
+        const float ms = (mx == neg_inf()) ? 0.f : mx;
+        st.clear();
+        st.m = mx;
+#pragma unroll 2
+        for (int s = 0; s < item.z; ++s) {
+          const float* p = p0 + (size_t)s * (D + 4);
+          const float2 ml = __ldcg(reinterpret_cast<const float2*>(p + D));
+          const float4 a0 = __ldcg(reinterpret_cast<const float4*>(p) + 2 * (lane % LPK));
+          const float4 a1 = __ldcg(reinterpret_cast<const float4*>(p) + 2 * (lane % LPK) + 1);
+          const float c = fast_exp2((ml.x - ms) * kLog2e);
+          st.l = fmaf(ml.y, c, st.l);
+          st.acc.v[0] = fmaf(a0.x, c, st.acc.v[0]);
+          st.acc.v[1] = fmaf(a0.y, c, st.acc.v[1]);
+          st.acc.v[2] = fmaf(a0.z, c, st.acc.v[2]);
+          st.acc.v[3] = fmaf(a0.w, c, st.acc.v[3]);
+          st.acc.v[4] = fmaf(a1.x, c, st.acc.v[4]);
+          st.acc.v[5] = fmaf(a1.y, c, st.acc.v[5]);
+          st.acc.v[6] = fmaf(a1.z, c, st.acc.v[6]);
+          st.acc.v[7] = fmaf(a1.w, c, st.acc.v[7]);
+        }
+        if (st.l > 0.f) store_row16<D, T>(st, m, l, O, r, lane);
+      }
+      return;
+    }
+    if ((int)blockIdx.x >= list_begin) block -= list_blocks;
+  }
+  if (threadIdx.x == 0) {
+    s_n_heavy = 0;
+    s_next = kRowWarps;
+  }
   __syncthreads();
-  const int64_t r = (int64_t)blockIdx.x * kRowWarps + warp;
-  if (r < n_rows) {
+  const int64_t first = block * rows_per_cta;
+  for (int i = warp; i < rows_per_cta && first + i < n_rows;) {  // warp-uniform
+    const int64_t r = first + i;
     const typename Cols::Row row = cols.open(r, row_begin + r);
     if (row.n <= 0) {
       if (Cols::kNanFillEmpty && use_nan && lane < LPK) {
         const uint32_t nn = Cvt16<T>::down(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
         *reinterpret_cast<uint4*>(O + (size_t)r * D + lane * 8) = make_uint4(nn, nn, nn, nn);
       }
-    } else if (row.n > kHeavyRowSlots) {
-      if (lane == 0) s_heavy[atomicAdd(&s_n_heavy, 1)] = warp;
+    } else if (row.n > (SLICED ? kSliceSlots : kHeavyRowSlots)) {
+      if (!SLICED && lane == 0) s_heavy[atomicAdd(&s_n_heavy, 1)] = i;
     } else {
       const Vec8 q = ldg8<T>(Q + (size_t)r * D + (lane % LPK) * 8);
       RowAcc8 st;
@@ -215,11 +344,16 @@ gather_rows16_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* 
       merge_groups16<LPK>(st);
       if (st.l > 0.f) store_row16<D, T>(st, m, l, O, r, lane);
     }
+    if (rows_per_cta <= kRowWarps) break;
+    int nxt = 0;
+    if (lane == 0) nxt = atomicAdd(&s_next, 1);
+    i = __shfl_sync(kFullMask, nxt, 0);
   }
+  if (SLICED) return;
   __syncthreads();
   const int n_heavy = s_n_heavy;  // uniform over the CTA
   for (int h = 0; h < n_heavy; ++h) {  // long rows: every warp of the CTA takes a share of the slots
-    const int64_t rh = (int64_t)blockIdx.x * kRowWarps + s_heavy[h];
+    const int64_t rh = first + s_heavy[h];
     const typename Cols::Row row = cols.open(rh, row_begin + rh);
     int64_t per = (row.n + kRowWarps - 1) / kRowWarps;
     per = (per + 31) / 32 * 32;

@@ -1,6 +1,7 @@
 // C ABI, 16-bit storage (float16 / bfloat16 Q, K, V, m, l, O): the native gather path for all six mask families.
 // Declared in include/spfa_b200.h under "16-bit tensors". Arithmetic is fp32; only loads and stores are 16-bit.
 #include <cmath>
+#include <type_traits>
 
 #include "capi_common.cuh"
 #include "gather_generic.cuh"
@@ -9,13 +10,56 @@
 
 namespace spfa {
 
+// Scratch of the sliced long rows: [count | items | done | part].
+inline unsigned int slice_cap(int64_t nnz) { return (unsigned int)(2 * (nnz / kSliceSlots) + 1); }
+inline size_t slice_scratch_bytes(int64_t nnz, int d) {
+  if (nnz <= kSliceSlots || nnz > (1LL << 37)) return 0;
+  const size_t cap = slice_cap(nnz);
+  return 256 + align_up(cap * sizeof(int4)) + align_up(cap * 4) + align_up(cap * (size_t)(d + 4) * 4);
+}
+inline RowSlices slice_view(char* ws, int64_t nnz, int d) {
+  RowSlices sl;
+  sl.cap = slice_cap(nnz);
+  sl.count = reinterpret_cast<unsigned int*>(ws);
+  sl.items = reinterpret_cast<int4*>(ws + 256);
+  sl.done = reinterpret_cast<unsigned int*>(ws + 256 + align_up(sl.cap * sizeof(int4)));
+  sl.part = reinterpret_cast<float*>(ws + 256 + align_up(sl.cap * sizeof(int4)) + align_up((size_t)sl.cap * 4));
+  return sl;
+}
+
+// `slices`: scratch for the long rows of an explicit mask (null: long rows are walked by their CTA).
 template <int D, class T, class Cols>
 int launch_gather16(const T* Q, const T* K, const T* V, T* m, T* l, T* O, const Cols& cols, int64_t row_begin,
-                    int64_t n_rows, int use_nan, cudaStream_t st) {
-  const int64_t blocks = (n_rows + kRowWarps - 1) / kRowWarps;
-  if (blocks > 0x7fffffffLL) return SPFA_ERR_TOO_LARGE;
-  gather_rows16_kernel<D, T, Cols><<<(unsigned)blocks, kRowWarps * 32, 0, st>>>(Q, K, V, m, l, O, cols, row_begin, n_rows,
-                                                                                use_nan, 1.0f / sqrtf((float)D));
+                    int64_t n_rows, int use_nan, cudaStream_t st, const RowSlices* slices = nullptr) {
+  const int per_cta = rows_per_cta_for(n_rows, 1);
+  const int64_t blocks = (n_rows + per_cta - 1) / per_cta;
+  if (blocks > 0x7fffffffLL - 1024) return SPFA_ERR_TOO_LARGE;
+  const float scale = 1.0f / sqrtf((float)D);
+  if constexpr (std::is_same<Cols, CsrCols>::value) {
+    if (slices) {
+      if (cudaMemsetAsync(slices->count, 0, 4, st) != cudaSuccess) return SPFA_ERR_LAUNCH;
+      row_slices_kernel<<<(unsigned)((n_rows + 255) / 256), 256, 0, st>>>(cols.row_off, n_rows, *slices);
+      const int wave = 148 * 6;  // resident CTAs of the gather kernel
+      const int list_begin = blocks < wave ? (int)blocks : wave;
+      const int list_blocks = (int)((slices->cap + kRowWarps - 1) / kRowWarps < (unsigned)wave ? (slices->cap + kRowWarps - 1) / kRowWarps : wave);
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)(blocks + list_blocks));
+      cfg.blockDim = dim3(kRowWarps * 32);
+      cfg.stream = st;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[0].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      if (cudaLaunchKernelEx(&cfg, gather_rows16_kernel<D, T, Cols, true>, Q, K, V, m, l, O, cols, row_begin, n_rows, use_nan,
+                             scale, per_cta, *slices, list_begin, list_blocks) != cudaSuccess)
+        return SPFA_ERR_LAUNCH;
+      g_launches.fetch_add(2);
+      return launch_status();
+    }
+  }
+  gather_rows16_kernel<D, T, Cols, false><<<(unsigned)blocks, kRowWarps * 32, 0, st>>>(
+      Q, K, V, m, l, O, cols, row_begin, n_rows, use_nan, scale, per_cta, RowSlices{}, 0, 0);
   g_launches.fetch_add(1);
   return launch_status();
 }
@@ -34,13 +78,13 @@ int launch_generic16(const T* Q, const T* K, const T* V, T* m, T* l, T* O, const
 // d in {32, 64, 128}: the specialised kernel; other multiples of 8: 128-bit pieces; anything else: scalar pieces.
 template <class T, class Cols>
 int dispatch16(int d, const T* Q, const T* K, const T* V, T* m, T* l, T* O, const Cols& cols, int64_t row_begin,
-               int64_t n_rows, int use_nan, cudaStream_t st) {
+               int64_t n_rows, int use_nan, cudaStream_t st, const RowSlices* slices = nullptr) {
   if (n_rows <= 0) return SPFA_OK;
   g_last_path.store(SPFA_PATH_GATHER);
   switch (d) {
-    case 32: return launch_gather16<32, T, Cols>(Q, K, V, m, l, O, cols, row_begin, n_rows, use_nan, st);
-    case 64: return launch_gather16<64, T, Cols>(Q, K, V, m, l, O, cols, row_begin, n_rows, use_nan, st);
-    case 128: return launch_gather16<128, T, Cols>(Q, K, V, m, l, O, cols, row_begin, n_rows, use_nan, st);
+    case 32: return launch_gather16<32, T, Cols>(Q, K, V, m, l, O, cols, row_begin, n_rows, use_nan, st, slices);
+    case 64: return launch_gather16<64, T, Cols>(Q, K, V, m, l, O, cols, row_begin, n_rows, use_nan, st, slices);
+    case 128: return launch_gather16<128, T, Cols>(Q, K, V, m, l, O, cols, row_begin, n_rows, use_nan, st, slices);
   }
   if (d % 8 == 0) return launch_generic16<T, 8, 4, Cols>(Q, K, V, m, l, O, cols, row_begin, n_rows, use_nan, d, st);
   return launch_generic16<T, 1, 32, Cols>(Q, K, V, m, l, O, cols, row_begin, n_rows, use_nan, d, st);
@@ -71,9 +115,17 @@ using namespace spfa;
 
 extern "C" {
 
+size_t spfa_csr_workspace_bytes_16(int64_t, int64_t nnz, int d) { return slice_scratch_bytes(nnz, d); }
+
 int spfa_csr_forward_16(int dtype, const void* Q, const void* K, const void* V, const uint64_t* row_off,
                         const uint32_t* col_ind, int64_t nnz, void* m, void* l, void* O, int64_t n_rows, int64_t Lk, int d,
                         int use_nan, void* stream) {
+  return spfa_csr_forward_16_ws(dtype, Q, K, V, row_off, col_ind, nnz, m, l, O, n_rows, Lk, d, use_nan, nullptr, 0, stream);
+}
+
+int spfa_csr_forward_16_ws(int dtype, const void* Q, const void* K, const void* V, const uint64_t* row_off,
+                           const uint32_t* col_ind, int64_t nnz, void* m, void* l, void* O, int64_t n_rows, int64_t Lk, int d,
+                           int use_nan, void* workspace, size_t workspace_bytes, void* stream) {
   int rc = check_common16(Q, K, V, m, l, O, d);
   if (rc) return rc;
   if (!row_off || n_rows < 0 || nnz < 0 || Lk <= 0 || Lk >= (1LL << 31)) return SPFA_ERR_BAD_ARG;
@@ -82,8 +134,12 @@ int spfa_csr_forward_16(int dtype, const void* Q, const void* K, const void* V, 
   return with_dtype16(dtype, [&](auto* tag) {
     using T = typename std::remove_pointer<decltype(tag)>::type;
     CsrCols cols{row_off, col_ind, Lk};
+    const size_t need = slice_scratch_bytes(nnz, d);
+    RowSlices sl{};
+    const bool sliced = need && check_workspace(workspace, workspace_bytes, need) == SPFA_OK;
+    if (sliced) sl = slice_view(static_cast<char*>(workspace), nnz, d);
     return dispatch16<T>(d, (const T*)Q, (const T*)K, (const T*)V, (T*)m, (T*)l, (T*)O, cols, 0, n_rows, use_nan,
-                         (cudaStream_t)stream);
+                         (cudaStream_t)stream, sliced ? &sl : nullptr);
   });
 }
 
@@ -108,7 +164,12 @@ int spfa_coo_forward_16(int dtype, const void* Q, const void* K, const void* V, 
   return with_dtype16(dtype, [&](auto* tag) {
     using T = typename std::remove_pointer<decltype(tag)>::type;
     CsrCols cols{ptr, col_ind, Lk};
-    return dispatch16<T>(d, (const T*)Q, (const T*)K, (const T*)V, (T*)m, (T*)l, (T*)O, cols, row_begin, n_rows, use_nan, st);
+    const size_t ptr_bytes = spfa_coo_min_workspace_bytes(n_rows), need = slice_scratch_bytes(nnz, d);
+    RowSlices sl{};
+    const bool sliced = need && workspace_bytes >= ptr_bytes + need;
+    if (sliced) sl = slice_view(static_cast<char*>(workspace) + ptr_bytes, nnz, d);
+    return dispatch16<T>(d, (const T*)Q, (const T*)K, (const T*)V, (T*)m, (T*)l, (T*)O, cols, row_begin, n_rows, use_nan, st,
+                         sliced ? &sl : nullptr);
   });
 }
 

@@ -331,11 +331,19 @@ int spfa_bigbird_forward_f32(const float* Q, const float* K, const float* V, flo
  * and calling the fp32 entry points, which is what the torch modules do. Arguments are those of the fp32 entry
  * points with `dtype` in front and without a path choice; pointers must be 16-byte aligned when d % 8 == 0, 2-byte
  * otherwise. Workspace: COO needs spfa_coo_min_workspace_bytes(n_rows), Global-no-local
- * spfa_global_no_local_workspace_bytes_16(L, n_global), the others none. */
+ * spfa_global_no_local_workspace_bytes_16(L, n_global), the others none. Rows of more than 256 entries of a CSR / COO mask
+ * are cut into slices that different warps walk when the caller gives scratch for it (long rows of a power-law graph
+ * otherwise set the length of the call): spfa_csr_workspace_bytes_16(n_rows, nnz, d) bytes, passed to
+ * spfa_csr_forward_16_ws, or behind the COO minimum in spfa_coo_forward_16's workspace. */
 typedef enum spfa_dtype { SPFA_DTYPE_F32 = 0, SPFA_DTYPE_F16 = 1, SPFA_DTYPE_BF16 = 2 } spfa_dtype;
 int spfa_csr_forward_16(int dtype, const void* Q, const void* K, const void* V,
                         const uint64_t* row_off, const uint32_t* col_ind, int64_t nnz,
                         void* m, void* l, void* O, int64_t n_rows, int64_t Lk, int d, int use_nan, void* stream);
+size_t spfa_csr_workspace_bytes_16(int64_t n_rows, int64_t nnz, int d);
+int spfa_csr_forward_16_ws(int dtype, const void* Q, const void* K, const void* V,
+                           const uint64_t* row_off, const uint32_t* col_ind, int64_t nnz,
+                           void* m, void* l, void* O, int64_t n_rows, int64_t Lk, int d, int use_nan,
+                           void* workspace, size_t workspace_bytes, void* stream);
 int spfa_coo_forward_16(int dtype, const void* Q, const void* K, const void* V,
                         const uint64_t* row_ind, const uint32_t* col_ind, int64_t nnz,
                         void* m, void* l, void* O, int64_t row_begin, int64_t n_rows, int64_t Lk, int d, int use_nan,

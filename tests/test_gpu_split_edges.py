@@ -1,0 +1,67 @@
+"""GPU: sizes at which a kernel changes how it splits its work (slice, tile and list limits), against the fp64 oracle."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import seeded_qkv
+
+pytestmark = pytest.mark.gpu
+
+# stored results: a few units in the last place of the 16-bit format for |O| <~ 4; fp32: sums of fp32 products
+TOL = {torch.float32: 1e-5, torch.float16: 2e-3, torch.bfloat16: 1.6e-2}
+
+
+@pytest.fixture()
+def capi(pkg):
+    c = pkg.capi
+    c.set_path(c.PATH_AUTO)
+    yield c
+    assert c.last_device_error() == 0
+
+
+def dev(x):
+    return torch.from_numpy(np.ascontiguousarray(x)).cuda()
+
+
+def state(n, d, dtype):
+    return (torch.full((n,), float("-inf"), device="cuda", dtype=dtype), torch.zeros(n, device="cuda", dtype=dtype),
+            torch.zeros(n, d, device="cuda", dtype=dtype))
+
+
+def close(st, want, tol, what):
+    m, l, O = (t.double().cpu().numpy() for t in st)
+    assert np.array_equal(np.isnan(O), np.isnan(want[2])), what
+    assert np.nanmax(np.abs(O - want[2])) <= tol, f"{what}: O {np.nanmax(np.abs(O - want[2])):.3e}"
+    fin = np.isfinite(want[0])
+    assert np.array_equal(np.isfinite(m), fin), what
+    np.testing.assert_allclose(m[fin], want[0][fin], rtol=4 * tol, atol=4 * tol, err_msg=what)
+    np.testing.assert_allclose(l, want[1], rtol=4 * tol, atol=1e-6, err_msg=what)
+
+
+def csr_of_lengths(lengths, Lk, seed):
+    """Distinct ascending random columns, `lengths[r]` of them in row r."""
+    rng = np.random.default_rng(seed)
+    off = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int64)
+    col = np.concatenate([np.sort(rng.choice(Lk, n, replace=False)) for n in lengths] + [[]]).astype(np.int32)
+    return off, col
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("d", [32, 64, 128])
+def test_16bit_rows_around_the_slice_length(capi, orc, dtype, d):
+    """Rows of one slice exactly, one entry more, several slices with a remainder, an empty row, twice on one state."""
+    Lk = 5000
+    lengths = [0, 1, 255, 256, 257, 512, 513, 4999, 31, 33, 2048, 0, 300] + [7] * 50 + [1025]
+    off, col = csr_of_lengths(lengths, Lk, d)
+    n = len(lengths)
+    Q, K, V = seeded_qkv(n, d, 11 + d, Lk=Lk)
+    q, k, v = (dev(x).to(dtype) for x in (Q, K, V))
+    Qr, Kr, Vr = (x.float().cpu().numpy() for x in (q, k, v))
+    want = orc.csr_forward(Qr, Kr, Vr, off, col, use_nan=True)
+    st = state(n, d, dtype)
+    capi.forward_16("csr", q, k, v, *st, row_off=dev(off), col_ind=dev(col), use_nan=True)
+    close(st, want, TOL[dtype], f"csr {dtype} d={d}")
+    rows = np.repeat(np.arange(n), lengths).astype(np.int64)
+    st = state(n, d, dtype)
+    capi.forward_16("coo", q, k, v, *st, row_ind=dev(rows), col_ind=dev(col), use_nan=True)
+    close(st, want, TOL[dtype], f"coo {dtype} d={d}")
