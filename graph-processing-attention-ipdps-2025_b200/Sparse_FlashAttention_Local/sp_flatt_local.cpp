@@ -27,6 +27,15 @@ torch::Tensor spfa_local_cuda_forward(torch::Tensor Q, torch::Tensor K, torch::T
                                            Q.size(0), at::cuda::getCurrentCUDAStream().stream()));
     return O;
   }
+  if (tiled_16_takes(Q, K, V, m, l, O, local_size_each_dir, 1)) {  // wide windows: 16-bit operands on the tensor cores
+    check_qkv_state_16(Q, K, V, m, l, O);
+    TORCH_CHECK(K.size(0) == Q.size(0), "implicit masks need K/V with as many rows as Q");
+    c10::cuda::CUDAGuard guard(Q.device());
+    raise_for_status(spfa_local_forward_tiled_16(dtype_code(Q), Q.data_ptr(), K.data_ptr(), V.data_ptr(), m.data_ptr(),
+                                                 l.data_ptr(), O.data_ptr(), Q.size(0), (int)Q.size(1), local_size_each_dir, 0,
+                                                 Q.size(0), at::cuda::getCurrentCUDAStream().stream()));
+    return O;
+  }
   if (needs_float32_copy(Q))
     return via_float32(Q, K, V, m, l, O, [&](torch::Tensor q, torch::Tensor k, torch::Tensor v, torch::Tensor mm,
                                              torch::Tensor ll, torch::Tensor oo) {

@@ -72,8 +72,8 @@ inline bool needs_float32_copy(const torch::Tensor& Q) {
 }
 
 // float16 / bfloat16 tensors have native entry points (16-bit loads and stores around fp32 arithmetic, gather path).
-// The bindings take them wherever the fp32 call would take the gather path as well; wide bands and long listed-key
-// strips, which the fp32 entry points run on the tensor cores, are converted instead (via_float32 below).
+// The bindings take them wherever the fp32 call would take the gather path as well; wide bands have tensor-core entry points
+// of their own (tiled_16_takes below); long listed-key strips are converted (via_float32 below).
 inline bool is_16bit(const torch::Tensor& Q) {
   return Q.scalar_type() == torch::kFloat16 || Q.scalar_type() == torch::kBFloat16;
 }
@@ -94,6 +94,21 @@ inline void check_qkv_state_16(const torch::Tensor& Q, const torch::Tensor& K, c
   TORCH_CHECK(K.size(1) == d && V.size(1) == d && O.size(1) == d, "K, V, O must have Q's embedded dimension");
   TORCH_CHECK(K.size(0) == V.size(0), "K and V must have the same number of rows");
   TORCH_CHECK(O.size(0) == L && m.size(0) == L && l.size(0) == L, "O, m, l must have Q's number of rows");
+}
+// The 16-bit tensor-core kernels take a call whose tensors TMA can address (16-byte aligned) and whose state overlaps none of
+// Q, K, V: a converted call reads all of its inputs before it writes, a direct one does not.
+inline bool tiled_16_takes(const torch::Tensor& Q, const torch::Tensor& K, const torch::Tensor& V, const torch::Tensor& m,
+                           const torch::Tensor& l, const torch::Tensor& O, int64_t w, int64_t stride) {
+  if (!is_16bit(Q) || Q.dim() != 2) return false;
+  c10::cuda::CUDAGuard guard(Q.device());
+  if (!spfa_tiled_16_usable(dtype_code(Q), (int)Q.size(1), w, stride)) return false;
+  auto at = [](const torch::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()); };
+  for (const torch::Tensor* t : {&Q, &K, &V, &O})
+    if (at(*t) & 15u) return false;
+  for (const torch::Tensor* out : {&m, &l, &O})
+    for (const torch::Tensor* in : {&Q, &K, &V})
+      if (at(*out) < at(*in) + in->nbytes() && at(*in) < at(*out) + out->nbytes()) return false;
+  return true;
 }
 inline bool tiled_d(int64_t d) { return d == 32 || d == 64 || d == 128; }
 

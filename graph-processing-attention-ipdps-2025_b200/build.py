@@ -68,6 +68,10 @@ def _check_band_kernel_registers(ptxas_log: str) -> None:
         name, nsub, regs = m.group(1), m.group(2), int(m.group(3))
         if regs != want[nsub]:
             raise RuntimeError(f"{name}: ptxas assigned {regs} registers, the setmaxnreg budgets need {want[nsub]}")
+    for m in re.finditer(r"Compiling entry function '(_ZN4spfa4tile21band16_forward_kernel[^']*)'.*?Used (\d+) registers",
+                         ptxas_log, flags=re.S):
+        if int(m.group(2)) != 128:
+            raise RuntimeError(f"{m.group(1)}: ptxas assigned {m.group(2)} registers, the setmaxnreg budgets need 128")
 
 
 def build_lib(force: bool = False, verbose: bool = False) -> str:

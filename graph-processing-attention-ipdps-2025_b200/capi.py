@@ -37,7 +37,7 @@ EXPORTS = (
     "spfa_dense_mask_offsets", "spfa_dense_mask_fill", "spfa_bigbird_workspace_bytes", "spfa_bigbird_forward_f32",
     "spfa_local_forward_batched_f32", "spfa_local_1d_dilated_forward_batched_f32", "spfa_local_2d_dilated_forward_batched_f32",
     "spfa_global_no_local_forward_batched_f32", "spfa_csr_forward_batched_f32", "spfa_coo_forward_batched_f32",
-    "spfa_csr_forward_16", "spfa_csr_forward_16_ws", "spfa_csr_workspace_bytes_16", "spfa_coo_forward_16", "spfa_local_forward_16", "spfa_local_1d_dilated_forward_16",
+    "spfa_csr_forward_16", "spfa_csr_forward_16_ws", "spfa_csr_workspace_bytes_16", "spfa_coo_forward_16", "spfa_tiled_16_usable", "spfa_local_forward_tiled_16", "spfa_local_1d_dilated_forward_tiled_16", "spfa_local_forward_16", "spfa_local_1d_dilated_forward_16",
     "spfa_local_2d_dilated_forward_16", "spfa_global_no_local_workspace_bytes_16", "spfa_global_no_local_forward_16",
     "spfa_csr_workspace_bytes_idx32", "spfa_csr_forward_f32_idx32", "spfa_coo_forward_f32_idx32", "spfa_coo_plan_build_idx32",
 )
@@ -100,6 +100,12 @@ def lib() -> ctypes.CDLL:
     L.spfa_local_forward_16.argtypes = [i32] + [vp] * 6 + [i64, i32, i64, i64, i64, vp]
     L.spfa_local_1d_dilated_forward_16.restype = i32
     L.spfa_local_1d_dilated_forward_16.argtypes = [i32] + [vp] * 6 + [i64, i32, i64, i64, i64, i64, vp]
+    L.spfa_tiled_16_usable.restype = i32
+    L.spfa_tiled_16_usable.argtypes = [i32, i32, i64, i64]
+    L.spfa_local_forward_tiled_16.restype = i32
+    L.spfa_local_forward_tiled_16.argtypes = L.spfa_local_forward_16.argtypes
+    L.spfa_local_1d_dilated_forward_tiled_16.restype = i32
+    L.spfa_local_1d_dilated_forward_tiled_16.argtypes = L.spfa_local_1d_dilated_forward_16.argtypes
     L.spfa_local_2d_dilated_forward_16.restype = i32
     L.spfa_local_2d_dilated_forward_16.argtypes = [i32] + [vp] * 6 + [i64, i32, i64, i64, i32, i64, i64, vp]
     L.spfa_global_no_local_workspace_bytes_16.restype = sz
@@ -463,9 +469,10 @@ def _t16(*ts):
 
 
 def forward_16(kind, Q, K, V, m, l, O, *, p0=0, p1=0, global_inds=None, row_off=None, row_ind=None, col_ind=None,
-               use_nan=False, row_begin=0, row_end=None):
+               use_nan=False, row_begin=0, row_end=None, tiled=False):
     """Native 16-bit forward of one mask family (`kind`: csr, coo, local, local_1d_dilated, local_2d_dilated,
-    global_no_local) on float16 / bfloat16 tensors: 16-bit loads and stores, fp32 arithmetic, gather path."""
+    global_no_local) on float16 / bfloat16 tensors: 16-bit loads and stores, fp32 arithmetic, gather path; `tiled` takes the
+    tensor-core kernel (local and local_1d_dilated)."""
     dev, code = _t16(Q, K, V, m, l, O)
     n_rows, d = Q.shape
     Lk = K.shape[0]
@@ -484,10 +491,11 @@ def forward_16(kind, Q, K, V, m, l, O, *, p0=0, p1=0, global_inds=None, row_off=
         else:
             L, row_end = _rows(Q, K, row_begin, row_end)
             if kind == "local":
-                rc = lib().spfa_local_forward_16(code, q, k, v, mm, ll, oo, L, d, int(p0), row_begin, row_end, st)
+                f = lib().spfa_local_forward_tiled_16 if tiled else lib().spfa_local_forward_16
+                rc = f(code, q, k, v, mm, ll, oo, L, d, int(p0), row_begin, row_end, st)
             elif kind == "local_1d_dilated":
-                rc = lib().spfa_local_1d_dilated_forward_16(code, q, k, v, mm, ll, oo, L, d, int(p0), int(p1), row_begin,
-                                                            row_end, st)
+                f = lib().spfa_local_1d_dilated_forward_tiled_16 if tiled else lib().spfa_local_1d_dilated_forward_16
+                rc = f(code, q, k, v, mm, ll, oo, L, d, int(p0), int(p1), row_begin, row_end, st)
             elif kind == "local_2d_dilated":
                 rc = lib().spfa_local_2d_dilated_forward_16(code, q, k, v, mm, ll, oo, L, d, int(p0), int(p1), int(use_nan),
                                                             row_begin, row_end, st)

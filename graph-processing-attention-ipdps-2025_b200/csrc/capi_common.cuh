@@ -20,6 +20,9 @@ struct PathCell {
 extern thread_local PathCell g_path;
 extern thread_local PathCell g_last_path;
 
+// Device address of the tiled kernels' error word (bounded waits record a code there); null if it cannot be had.
+int* tile_error_word();
+
 inline size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 inline bool aligned4(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 3u) == 0; }

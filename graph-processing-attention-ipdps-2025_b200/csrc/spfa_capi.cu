@@ -470,6 +470,15 @@ int launch_row_pointers(const IdxT* row_ind, int64_t nnz, int64_t row_begin, int
 
 }  // namespace spfa
 
+namespace spfa {
+
+int* tile_error_word() {
+  int* err = nullptr;
+  return cudaGetSymbolAddress(reinterpret_cast<void**>(&err), g_tile_error) == cudaSuccess ? err : nullptr;
+}
+
+}  // namespace spfa
+
 using namespace spfa;
 
 namespace spfa {

@@ -12,6 +12,7 @@
 
 #include "../../include/spfa_b200.h"
 #include "gather_kernels.cuh"
+#include "tensor_map.cuh"
 #include "tile_kernels_sm100.cuh"
 
 namespace spfa {
@@ -56,23 +57,6 @@ inline int tile_ctas_per_sm(int d) { return d == 128 ? TileCfg<128>::kCtasPerSm 
 
 // Error word of the tiled kernels (bounded waits record a code here). One per device context.
 __device__ int g_tile_error;
-
-typedef CUresult (*TensorMapEncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                           const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                           CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                           CUtensorMapFloatOOBfill);
-
-inline TensorMapEncodeTiledFn tensor_map_encoder() {
-  static TensorMapEncodeTiledFn fn = []() -> TensorMapEncodeTiledFn {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      return nullptr;
-    return reinterpret_cast<TensorMapEncodeTiledFn>(p);
-  }();
-  return fn;
-}
 
 // [rows, d] fp32 matrix with a row pitch of `pitch_bytes`, fetched as boxes of box_rows x 32 floats with the
 // 128-byte swizzle the MMA descriptors expect (16-byte units for K-major operands, 32-byte units for the

@@ -327,9 +327,8 @@ int spfa_bigbird_forward_f32(const float* Q, const float* K, const float* V, flo
  * points read and write such tensors directly -- half the bytes of an fp32 call on the gather path, where HBM traffic
  * is the limit -- and compute in fp32 (the reference accumulates in half), so results are at least as accurate as
  * its own. bfloat16 is additive. They always take the warp-per-row gather path (any d from 1 to 1024; d in
- * {32, 64, 128} has specialised kernels); wide banded masks on 16-bit inputs are better served by converting to fp32
- * and calling the fp32 entry points, which is what the torch modules do. Arguments are those of the fp32 entry
- * points with `dtype` in front and without a path choice; pointers must be 16-byte aligned when d % 8 == 0, 2-byte
+ * {32, 64, 128} has specialised kernels); wide banded masks are better served by the *_tiled_16 entry points below.
+ * Arguments are those of the fp32 entry points with `dtype` in front and without a path choice; pointers must be 16-byte aligned when d % 8 == 0, 2-byte
  * otherwise. Workspace: COO needs spfa_coo_min_workspace_bytes(n_rows), Global-no-local
  * spfa_global_no_local_workspace_bytes_16(L, n_global), the others none. Rows of more than 256 entries of a CSR / COO mask
  * are cut into slices that different warps walk when the caller gives scratch for it (long rows of a power-law graph
@@ -356,6 +355,16 @@ int spfa_local_1d_dilated_forward_16(int dtype, const void* Q, const void* K, co
 int spfa_local_2d_dilated_forward_16(int dtype, const void* Q, const void* K, const void* V, void* m, void* l, void* O,
                                      int64_t L, int d, int64_t block_size, int64_t dil_factor, int use_nan,
                                      int64_t row_begin, int64_t row_end, void* stream);
+/* Banded masks on the tensor cores: d in {32, 64, 128}, dil_factor < 16. Probabilities stay fp32 (two 16-bit terms each in
+ * the second product). As on the fp32 tiled path a key outside a row's window meets its V row with weight 0, so infinities
+ * and NaN in V reach rows of the same 64-key tiles. spfa_tiled_16_usable: 1 where the torch modules take these entry points
+ * (window of at least 32, stride = dil_factor + 1 up to 16, path selector not on SPFA_PATH_GATHER), else 0. */
+int spfa_tiled_16_usable(int dtype, int d, int64_t local_size_each_dir, int64_t stride);
+int spfa_local_forward_tiled_16(int dtype, const void* Q, const void* K, const void* V, void* m, void* l, void* O,
+                                int64_t L, int d, int64_t local_size_each_dir, int64_t row_begin, int64_t row_end, void* stream);
+int spfa_local_1d_dilated_forward_tiled_16(int dtype, const void* Q, const void* K, const void* V, void* m, void* l, void* O,
+                                           int64_t L, int d, int64_t local_size_each_dir, int64_t dil_factor,
+                                           int64_t row_begin, int64_t row_end, void* stream);
 size_t spfa_global_no_local_workspace_bytes_16(int64_t L, int64_t n_global);
 int spfa_global_no_local_forward_16(int dtype, const void* Q, const void* K, const void* V, void* m, void* l, void* O,
                                     const int32_t* global_inds, int64_t n_global, int64_t L, int d,

@@ -65,3 +65,29 @@ def test_16bit_rows_around_the_slice_length(capi, orc, dtype, d):
     st = state(n, d, dtype)
     capi.forward_16("coo", q, k, v, *st, row_ind=dev(rows), col_ind=dev(col), use_nan=True)
     close(st, want, TOL[dtype], f"coo {dtype} d={d}")
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("d", [32, 64, 128])
+@pytest.mark.parametrize("L,w,dil,lo,hi", [
+    (33, 32, 0, 0, 33), (64, 63, 0, 0, 64), (128, 40, 0, 0, 128), (129, 32, 0, 0, 129), (700, 33, 0, 0, 700),
+    (1000, 999, 0, 0, 1000), (1003, 200, 0, 131, 777), (515, 32, 2, 0, 515), (1201, 100, 6, 37, 1200), (300, 299, 15, 0, 300)])
+def test_16bit_band_tiles(capi, orc, dtype, d, L, w, dil, lo, hi):
+    """Tensor-core band on 16-bit tensors: ragged tiles, one row beyond a tile, row ranges, residue classes; a second call on
+    the same state (old rows are merged) and a state with one dead row among fresh ones. The oracle sees the rounded
+    tensors; the result's error is the rounding of the stored values."""
+    kind, p = ("local_1d_dilated", (w, dil)) if dil else ("local", (w, 0))
+    q, k, v = (dev(x).to(dtype) for x in seeded_qkv(L, d, 5 + d))
+    Qr, Kr, Vr = (x.float().cpu().numpy() for x in (q, k, v))
+    want = orc.implicit_forward(kind, Qr[lo:hi], Kr, Vr, *p, row_begin=lo, row_end=hi)
+    st = state(hi - lo, d, dtype)
+    st[2].fill_(3.0)  # l = 0: what O holds does not count
+    run = lambda s: capi.forward_16(kind, q[lo:hi], k, v, *s, p0=p[0], p1=p[1], row_begin=lo, row_end=hi, tiled=True)
+    run(st)
+    close(st, want, TOL[dtype], f"{kind} {dtype} L={L} d={d} w={w} dil={dil}")
+    # the same keys once more: m and O stay, l doubles; rows whose state was emptied in between give the first result again
+    st[0][::5], st[1][::5] = float("-inf"), 0.0
+    run(st)
+    l2 = 2 * want[1]
+    l2[::5] = want[1][::5]
+    close(st, (want[0], l2, want[2]), 2 * TOL[dtype], f"{kind} again")
