@@ -79,24 +79,6 @@ __device__ __forceinline__ void mma16_ts(uint32_t d_tmem, uint32_t a_tmem, uint6
       : "memory");
 }
 
-// Two fp32 lanes in one 64-bit register: half the issue slots of the scalar forms.
-__device__ __forceinline__ uint64_t pack2(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x)); }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
 template <class T> struct Half16;
 template <> struct Half16<__half> {
   static __device__ __forceinline__ uint32_t down(float a, float b) {
@@ -293,19 +275,21 @@ band16_forward_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       for (int c = 0; c < NC; ++c)
         if (cls[c] != 0) tmem_ld32(tS + c * 32, sr[c]);
       tc_wait_ld();
+      // masked columns become -inf once; the code after is the same for every chunk class
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+        if (cls[c] == 1) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) sr[c][e] = ((vmask[c] >> e) & 1u) ? sr[c][e] : 0xff800000u;
+        }
       float mx[4] = {neg_inf(), neg_inf(), neg_inf(), neg_inf()};
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        if (cls[c] == 2) {
+      for (int c = 0; c < NC; ++c)
+        if (cls[c] != 0) {
 #pragma unroll
           for (int e = 0; e < 32; e += 2)
             mx[(e >> 1) & 3] = fmaxf(fmaxf(mx[(e >> 1) & 3], __uint_as_float(sr[c][e])), __uint_as_float(sr[c][e + 1]));
-        } else if (cls[c] == 1) {
-#pragma unroll
-          for (int e = 0; e < 32; ++e)
-            mx[e & 3] = fmaxf(mx[e & 3], ((vmask[c] >> e) & 1u) ? __uint_as_float(sr[c][e]) : neg_inf());
         }
-      }
       const float t_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sc;  // sc > 0
       m_true = fmaxf(m_true, t_max);
       const bool move = t_max > shift + kShiftSlack;
@@ -345,11 +329,7 @@ band16_forward_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         for (int e = 0; e < 16; ++e) {
           float x0, x1;
           unpack2(fma2(pack2(__uint_as_float(sr[c][2 * e]), __uint_as_float(sr[c][2 * e + 1])), sc2, ns2), x0, x1);
-          float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
-          if (cls[c] == 1) {
-            p0 = ((vmask[c] >> (2 * e)) & 1u) ? p0 : 0.f;
-            p1 = ((vmask[c] >> (2 * e + 1)) & 1u) ? p1 : 0.f;
-          }
+          const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
           const uint64_t p = pack2(p0, p1);
           l2[e & 1] = add2(l2[e & 1], p);
           const uint32_t h = H::down(p0, p1);

@@ -237,6 +237,24 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
                : "memory");
 }
 
+// Two fp32 lanes in one 64-bit register: half the issue slots of the scalar forms.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 __device__ __forceinline__ uint32_t to_tf32(float x) {
   uint32_t y;
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(y) : "f"(x));
@@ -841,19 +859,24 @@ band_forward_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       for (int c = 0; c < NC; ++c)
         if (cls[c] != 0) tmem_ld32(tS + c * 32, sr[c]);
       tc_wait_ld();
-      // ---- row maximum over the valid columns ----
+      // ---- masked columns become -inf once, in the chunks that have some; everything after is the same straight code for
+      //      every chunk class (exp2 of -inf is the 0 a masked pair contributes), which keeps the loop small enough for the
+      //      instruction cache ----
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+        if (cls[c] == 1) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) sr[c][e] = ((vmask[c] >> e) & 1u) ? sr[c][e] : 0xff800000u;
+        }
+      // ---- row maximum ----
       float mx[4] = {neg_inf(), neg_inf(), neg_inf(), neg_inf()};
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        if (cls[c] == 2) {
+      for (int c = 0; c < NC; ++c)
+        if (cls[c] != 0) {
 #pragma unroll
-          for (int e = 0; e < 32; ++e) mx[e & 3] = fmaxf(mx[e & 3], __uint_as_float(sr[c][e]));
-        } else if (cls[c] == 1) {
-#pragma unroll
-          for (int e = 0; e < 32; ++e)
-            mx[e & 3] = fmaxf(mx[e & 3], ((vmask[c] >> e) & 1u) ? __uint_as_float(sr[c][e]) : neg_inf());
+          for (int e = 0; e < 32; e += 2)
+            mx[(e >> 1) & 3] = fmaxf(fmaxf(mx[(e >> 1) & 3], __uint_as_float(sr[c][e])), __uint_as_float(sr[c][e + 1]));
         }
-      }
       const float t_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sc;  // sc > 0
       m_true = fmaxf(m_true, t_max);
       // ---- move the reference if this row outgrew it (always on the row's first valid tile) ----
@@ -887,23 +910,18 @@ band_forward_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       const float neg_shift = (shift == neg_inf()) ? 0.f : -shift;
       // ---- P = exp2(S*sc - shift) truncated to tf32 (the bits the MMA reads); the row sum adds the
       //      truncated values so that P / l stays exactly normalised; P goes back over S ----
-      float ls[4] = {0.f, 0.f, 0.f, 0.f};
+      const uint64_t sc2 = pack2(sc, sc), ns2 = pack2(neg_shift, neg_shift);
+      uint64_t ls2[2] = {0ull, 0ull};  // four partial sums, two to a register pair
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
-        if (cls[c] == 2) {
+        if (cls[c] != 0) {
 #pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            const uint32_t pb = __float_as_uint(fast_exp2(fmaf(__uint_as_float(sr[c][e]), sc, neg_shift))) & 0xffffe000u;
-            ls[e & 3] += __uint_as_float(pb);
-            sr[c][e] = pb;
-          }
-        } else if (cls[c] == 1) {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            uint32_t pb = __float_as_uint(fast_exp2(fmaf(__uint_as_float(sr[c][e]), sc, neg_shift))) & 0xffffe000u;
-            pb = ((vmask[c] >> e) & 1u) ? pb : 0u;
-            ls[e & 3] += __uint_as_float(pb);
-            sr[c][e] = pb;
+          for (int e = 0; e < 32; e += 2) {
+            float x0, x1;
+            unpack2(fma2(pack2(__uint_as_float(sr[c][e]), __uint_as_float(sr[c][e + 1])), sc2, ns2), x0, x1);
+            sr[c][e] = __float_as_uint(fast_exp2(x0)) & 0xffffe000u;
+            sr[c][e + 1] = __float_as_uint(fast_exp2(x1)) & 0xffffe000u;
+            ls2[(e >> 1) & 1] = add2(ls2[(e >> 1) & 1], pack2(__uint_as_float(sr[c][e]), __uint_as_float(sr[c][e + 1])));
           }
         } else {
 #pragma unroll
@@ -911,6 +929,9 @@ band_forward_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
         tmem_st32(tS + c * 32, sr[c]);
       }
+      float ls[4];
+      unpack2(ls2[0], ls[0], ls[1]);
+      unpack2(ls2[1], ls[2], ls[3]);
       tc_wait_st();
       tc_fence_before();
       mbar_arrive(bar(B_PREADY + sb));
