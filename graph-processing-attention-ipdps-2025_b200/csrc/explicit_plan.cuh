@@ -383,6 +383,60 @@ explicit_plan_kernel(const uint64_t* __restrict__ row_off, const uint32_t* __res
   }
   __syncthreads();
   const int nt = s_nt;
+  // A block without dense tiles (scattered masks): its residual list is its stretch of the column array as it is, provided
+  // that every column is a key and the offsets ascend. It is copied entry by entry; the walk below, which takes a row at a
+  // time and looks every entry up, spends a 128-entry step on a row of 32. The order check counts descents over the stretch
+  // and takes off those that fall between two rows. (131072 rows of 32 random keys: 59.6 -> 21.7 us.)
+  if (nt == 0 && !__syncthreads_or(tid < nr && s_off[tid] > s_off[tid + 1])) {
+    bool bad = false;
+    const int64_t a = (int64_t)s_off[0], z = (int64_t)s_off[nr];
+    int descents = 0;
+    for (int64_t p0 = a; p0 < z; p0 += 4 * kPlanThreads) {
+      uint32_t c[4], before[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int64_t p = p0 + k * kPlanThreads + tid;
+        c[k] = before[k] = 0u;
+        if (p < z) {
+          c[k] = __ldg(col + p);
+          if (p > a) before[k] = __ldg(col + p - 1);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int64_t p = p0 + k * kPlanThreads + tid;
+        if (p >= z) break;
+        bad = bad || c[k] >= Lk32;
+        descents += before[k] > c[k];
+        plan.res_col[p] = c[k];
+      }
+    }
+    if (!__syncthreads_or(bad)) {
+      if (tid < nr) {
+        const int64_t ra = (int64_t)s_off[tid], rz = (int64_t)s_off[tid + 1];
+        const uint32_t n = (uint32_t)(rz - ra);
+        if (n > 0 && ra > a) descents -= __ldg(col + ra - 1) > __ldg(col + ra);
+        plan.res_cnt[r0 + tid] = n;
+        if (n > (uint32_t)kListedRowSlots) list_long_row(plan, (int)(r0 + tid), n);
+      }
+      descents = __reduce_add_sync(kFullMask, descents);
+      if (lane == 0 && descents) atomicAdd(&s_in_dense, descents);  // 0 until here: no tile is dense
+      if (use_nan)
+        for (int rl = warp; rl < nr; rl += kPlanWarps)
+          if (s_off[rl] == s_off[rl + 1]) {
+            const float nn = __int_as_float(0x7fc00000);
+            for (int i = lane * 4; i < d; i += 128)
+              *reinterpret_cast<float4*>(O + (size_t)(r0 + rl) * d + i) = make_float4(nn, nn, nn, nn);
+          }
+      __syncthreads();
+      if (tid == 0) {
+        if (s_in_dense) *plan.unsorted = 1u;
+        plan.rb_nt[b] = 0;
+        plan.rb_moff[b] = 0;
+      }
+      return;
+    }
+  }
   if (tid < nt) atomicAdd(&s_in_dense, (int)count_of(s_sel[tid]));
   __syncthreads();  // the histogram is dead from here on: its storage becomes the masks
   // A block whose entries lie almost all in dense tiles (block-structured masks) is walked with a warp-level shortcut

@@ -374,6 +374,16 @@ band_forward_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
   }
 
+  if (EXPL) {  // no dense tile in any block of this CTA (scattered masks): nothing to set up, its rows are not touched
+    bool some = false;
+#pragma unroll
+    for (int x = 0; x < NSUB; ++x) some = some || nt_early[x] > 0;
+    if (!some) {
+      if ((prm.overlap & 2) && threadIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+      return;
+    }
+  }
+
   // ---- tile geometry (uniform across the CTA) ----
   const int64_t uq0 = prm.u_q_first + (int64_t)blockIdx.x * kQRows;  // first query u of this CTA
   const int64_t uq_end = prm.u_q_first + prm.n_q;                    // one past the last valid query u

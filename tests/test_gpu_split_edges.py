@@ -91,3 +91,33 @@ def test_16bit_band_tiles(capi, orc, dtype, d, L, w, dil, lo, hi):
     l2 = 2 * want[1]
     l2[::5] = want[1][::5]
     close(st, (want[0], l2, want[2]), 2 * TOL[dtype], f"{kind} again")
+
+
+@pytest.mark.parametrize("d", [32, 64, 128])
+@pytest.mark.parametrize("fault", ["none", "unsorted", "beyond"])
+def test_scattered_blocks_of_an_explicit_mask(capi, orc, d, fault):
+    """Row blocks without a dense tile are copied whole: empty rows at block ends, rows around the listing (128) and slicing
+    (1024) limits, a row whose last column exceeds the next row's first; with a row out of order or a column beyond the keys
+    (dropped) in the second block; then the same plan over two key ranges."""
+    Lk = 200000
+    lengths = [0] + [5] * 60 + [127, 128, 129, 1023, 1024, 1025, 2500] + [40] * 59 + [0] + [33] * 70 + [0] * 3 + [1] * 72
+    off, col = csr_of_lengths(lengths, Lk, d)
+    n, at = len(lengths), int(off[150])
+    assert n > 256
+    if fault == "unsorted":
+        col[at], col[at + 1] = col[at + 1], col[at]
+    if fault == "beyond":
+        col[at] = Lk + 7
+    Q, K, V = seeded_qkv(n, d, 3 + d, Lk=Lk)
+    want = orc.csr_forward(Q, K, V, off, col, use_nan=True)
+    q, k, v = dev(Q), dev(K), dev(V)
+    capi.set_path(capi.PATH_TILED)
+    st = state(n, d, torch.float32)
+    capi.csr_forward(q, k, v, dev(off), dev(col), *st, use_nan=True)
+    assert capi.last_path() == capi.PATH_TILED and capi.last_csr_dense_tiles() == 0
+    close(st, want, TOL[torch.float32], f"one call, d={d}, {fault}")
+    plan = capi.csr_plan(dev(off), dev(col), Lk, d)
+    st = state(n, d, torch.float32)
+    capi.planned_forward_keys(q, k, v, *st, plan, 0, 64 * 1500, use_nan=True)
+    capi.planned_forward_keys(q, k, v, *st, plan, 64 * 1500, Lk)
+    close(st, want, TOL[torch.float32], f"two ranges, d={d}, {fault}")
