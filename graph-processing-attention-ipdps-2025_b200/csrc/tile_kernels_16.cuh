@@ -36,7 +36,7 @@ struct Band16Params {
 
 template <int D>
 struct Plan16 {
-  static constexpr int kThreads = 256, kRegsLaunch = 128, kRegsSoftmax = 208, kRegsAux = 48;
+  static constexpr int kThreads = 256, kRegsLaunch = 128, kRegsSoftmax = 176, kRegsAux = 80;
   static_assert(kRegsSoftmax * 128 + kRegsAux * 128 <= kRegsLaunch * kThreads, "setmaxnreg budgets exceed the launch pool");
   static constexpr int BN = 64, NS = (D == 128) ? 2 : 3;           // keys per tile, K and V stages
   static constexpr int kRowBytes = (D * 2 < 128) ? D * 2 : 128;    // one swizzled row of a chunk
@@ -178,46 +178,55 @@ band16_forward_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         ok = load(&tmV, P::kOffV, B_VFULL, B_VEMPTY, j);
         if (ok && j + NS < nT) ok = load(&tmK, P::kOffK, B_KFULL, B_KEMPTY, j + NS);
       }
-    } else if (warp == 5 && lane == 0) {
+    } else if (warp == 5) {
       // =============================== MMA issuer ===============================
+      const bool el = elect_one();
+      auto wait = [&](int b, uint32_t parity, int code) -> bool {
+        return __all_sync(kFullMask, mbar_wait(bar(b), parity, abort_flag, err, code));
+      };
       constexpr uint32_t kIdescS = idesc_16<T>(128, BN, 0);
       constexpr uint32_t kIdescO = idesc_16<T>(128, D, 1);
-      bool ok = mbar_wait(bar(B_QFULL), 0, abort_flag, err, 211);
+      bool ok = wait(B_QFULL, 0, 211);
       const uint64_t qd = smem_desc(sbase + P::kOffQ, 16, 8 * P::kRowBytes, P::kLayout);
       auto issue_S = [&](int j) -> bool {
         if (j >= nT) return true;
         const int st = j % NS;
-        if (!mbar_wait(bar(B_KFULL + st), (uint32_t)((j / NS) & 1), abort_flag, err, 212)) return false;
+        if (!wait(B_KFULL + st, (uint32_t)((j / NS) & 1), 212)) return false;
         tc_fence_after();
         const uint64_t kd = smem_desc(sbase + P::kOffK + st * P::kStageBytes, 16, 8 * P::kRowBytes, P::kLayout);
+        if (el) {
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {  // 16 elements (32 bytes) of the contraction per MMA
-          const int c = kk * 16 / P::kCols, in = kk * 32 % P::kRowBytes;
-          mma16_ss(tmem + P::kColS + BN * (j & 1), qd + (uint64_t)((c * P::kQChunkBytes + in) >> 4),
-                   kd + (uint64_t)((c * P::kKVChunkBytes + in) >> 4), kIdescS, kk ? 1u : 0u);
+          for (int kk = 0; kk < D / 16; ++kk) {  // 16 elements (32 bytes) of the contraction per MMA
+            const int c = kk * 16 / P::kCols, in = kk * 32 % P::kRowBytes;
+            mma16_ss(tmem + P::kColS + BN * (j & 1), qd + (uint64_t)((c * P::kQChunkBytes + in) >> 4),
+                     kd + (uint64_t)((c * P::kKVChunkBytes + in) >> 4), kIdescS, kk ? 1u : 0u);
+          }
+          tc_commit(bar(B_SREADY + (j & 1)));
+          tc_commit(bar(B_KEMPTY + st));
         }
-        tc_commit(bar(B_SREADY + (j & 1)));
-        tc_commit(bar(B_KEMPTY + st));
+        __syncwarp();
         return true;
       };
       ok = ok && issue_S(0) && issue_S(1);
       for (int j = 0; j < nT && ok; ++j) {
         const int st = j % NS;
-        ok = mbar_wait(bar(B_PREADY + (j & 1)), (uint32_t)((j >> 1) & 1), abort_flag, err, 213) &&
-             mbar_wait(bar(B_VFULL + st), (uint32_t)((j / NS) & 1), abort_flag, err, 214);
+        ok = wait(B_PREADY + (j & 1), (uint32_t)((j >> 1) & 1), 213) && wait(B_VFULL + st, (uint32_t)((j / NS) & 1), 214);
         if (!ok) break;
         tc_fence_after();
         // 16 keys per MMA = two 8-row swizzle groups; pieces of kCols dimensions are kKVChunkBytes apart
         const uint64_t vd = smem_desc(sbase + P::kOffV + st * P::kStageBytes, P::kKVChunkBytes, 8 * P::kRowBytes, P::kLayout);
         const uint32_t a_t = tmem + P::kColS + BN * (j & 1);
+        if (el) {
 #pragma unroll
-        for (int part = 0; part < 2; ++part)
+          for (int part = 0; part < 2; ++part)
 #pragma unroll
-          for (int kk = 0; kk < BN / 16; ++kk)
-            mma16_ts(tmem + P::kColO, a_t + part * (BN / 2) + kk * 8, vd + (uint64_t)((kk * 16 * P::kRowBytes) >> 4), kIdescO,
-                     (part | kk) ? 1u : (j > 0 ? 1u : 0u));
-        tc_commit(bar(B_OREADY + (j & 1)));
-        tc_commit(bar(B_VEMPTY + st));
+            for (int kk = 0; kk < BN / 16; ++kk)
+              mma16_ts(tmem + P::kColO, a_t + part * (BN / 2) + kk * 8, vd + (uint64_t)((kk * 16 * P::kRowBytes) >> 4), kIdescO,
+                       (part | kk) ? 1u : (j > 0 ? 1u : 0u));
+          tc_commit(bar(B_OREADY + (j & 1)));
+          tc_commit(bar(B_VEMPTY + st));
+        }
+        __syncwarp();
         ok = issue_S(j + 2);  // its S buffer is free once the PVs above are queued (the pipe runs them in order)
       }
     }

@@ -8,7 +8,7 @@
 // for d = 128, where one CTA interleaves its two sub-tiles on the tensor pipe. Roles (128 * NSUB + 128 threads):
 //   warps 0 .. 4 NSUB-1  softmax groups, one per sub-tile: thread t <-> query row t <-> TMEM lane t
 //   next warp            TMA producer (one elected lane) + TMEM allocation
-//   next warp            MMA issuer (one elected lane)
+//   next warp            MMA issuer (converged; one elected lane issues)
 //   last two warps       idle (they complete the last warpgroup so registers can be re-balanced with setmaxnreg)
 // Per key tile j and sub-tile X (S has two TMEM buffers per sub-tile, used alternately):
 //   S_X = Q_X K_j^T      tcgen05.mma kind::tf32, A = Q_X (smem, K-major), B = K_j (smem, K-major), D in TMEM;
@@ -48,14 +48,16 @@ namespace tile {
 // assigns under __launch_bounds__(kThreads, kCtasPerSm)). setmaxnreg.inc BLOCKS until the CTA's pool can
 // satisfy it and has no timeout, so the two budgets must fit in the pool the launch allocated -- otherwise
 // the softmax groups would wait forever. The host re-checks this against cudaFuncGetAttributes.
+// The split is the one at which neither side spills: with 208 / 48 and 216 / 72 it was the issuing and loading warps that
+// did (up to 276 bytes), inside the loops every key tile waits for.
 template <int NSUB>
 struct Geo {
   static constexpr int kThreads = 128 * NSUB + 128;
   static constexpr int kQRows = 128 * NSUB;
   static constexpr int kCtasPerSm = (NSUB == 1) ? 2 : 1;
   static constexpr int kRegsLaunch = (NSUB == 1) ? 128 : 168;
-  static constexpr int kRegsSoftmax = (NSUB == 1) ? 208 : 216;
-  static constexpr int kRegsAux = (NSUB == 1) ? 48 : 72;
+  static constexpr int kRegsSoftmax = (NSUB == 1) ? 160 : 192;
+  static constexpr int kRegsAux = (NSUB == 1) ? 96 : 120;
   static constexpr int kSoftmaxWarps = 4 * NSUB;
   static_assert(kRegsSoftmax * 128 * NSUB + kRegsAux * 128 <= kRegsLaunch * kThreads,
                 "setmaxnreg budgets exceed the launch pool");
@@ -183,6 +185,15 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// One lane of a converged warp. The issuing warp stays converged and only the tcgen05 instructions are predicated on the
+// elected lane, so that descriptors live in uniform registers: under a divergent `lane == 0` branch every operand was moved
+// there on its own and an MMA took 90-110 cycles to issue where the tensor pipe needs 32-64 (cycle stamps, d = 128).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
 
 // D[tmem] (+)= A[smem desc] * B[smem desc]
 __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
@@ -614,10 +625,15 @@ band_forward_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
   } else if (warp == W_MMA) {
     // =============================== MMA issuer ===============================
-    if (lane == 0) {
+    {
+      const bool el = elect_one();
+      // all lanes wait, so that the warp leaves a failed wait as one
+      auto wait = [&](int b, uint32_t parity, int code) -> bool {
+        return __all_sync(kFullMask, mbar_wait(bar(b), parity, abort_flag, err, code));
+      };
       constexpr uint32_t kIdescS = idesc_tf32(128, BN, 0);
       constexpr uint32_t kIdescO = idesc_tf32(128, D, 1);
-      bool ok = (nT > 0) && mbar_wait(bar(B_QFULL), 0, abort_flag, err, 201);
+      bool ok = (nT > 0) && wait(B_QFULL, 0, 201);
       // Descriptors are built once per operand tile; each MMA only adds a compile-time offset to the
       // 14-bit start-address field (shared memory is < 256 KB, so the field cannot carry out).
       // S of a sub-tile's it-th key tile goes to its S buffer it & 1; it is issued two tiles ahead of the
@@ -628,13 +644,16 @@ band_forward_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const uint64_t qd = smem_desc(sbase + P::kOffQ + x * P::kChunks * P::kQChunkBytes, 16, 1024, kLayoutSw128);
         const uint64_t kd = smem_desc(sbase + P::kOffK + st * P::kKVStageBytes, 16, 1024, kLayoutSw128);
         const uint32_t d_t = tmem + P::kColS + BN * sb;
+        if (el) {
 #pragma unroll
-        for (int c = 0; c < P::kChunks; ++c)
+          for (int c = 0; c < P::kChunks; ++c)
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            mma_ss(d_t, qd + (uint64_t)((c * P::kQChunkBytes + kk * 32) >> 4),
-                   kd + (uint64_t)((c * P::kKVChunkBytes + kk * 32) >> 4), kIdescS, (c | kk) ? 1u : 0u);
-        tc_commit(bar(B_SREADY + sb));
+            for (int kk = 0; kk < 4; ++kk)
+              mma_ss(d_t, qd + (uint64_t)((c * P::kQChunkBytes + kk * 32) >> 4),
+                     kd + (uint64_t)((c * P::kKVChunkBytes + kk * 32) >> 4), kIdescS, (c | kk) ? 1u : 0u);
+          tc_commit(bar(B_SREADY + sb));
+        }
+        __syncwarp();
       };
       auto issue_PV = [&](int x, int j) {
         const int st = j % NSV;
@@ -645,10 +664,13 @@ band_forward_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const uint32_t a_t = tmem + P::kColS + BN * sb;
         const uint32_t d_t = tmem + P::kColO + D * x;
         const uint32_t first = (it > 0) ? 1u : 0u;  // O accumulates in TMEM across the key tiles of a sub-tile
+        if (el) {
 #pragma unroll
-        for (int kk = 0; kk < BN / 8; ++kk)
-          mma_ts(d_t, a_t + kk * 8, vd + (uint64_t)((kk * 1024) >> 4), kIdescO, kk > 0 ? 1u : first);
-        tc_commit(bar(B_OREADY + sb));  // tiles alternate between two barriers, like the S buffers
+          for (int kk = 0; kk < BN / 8; ++kk)
+            mma_ts(d_t, a_t + kk * 8, vd + (uint64_t)((kk * 1024) >> 4), kIdescO, kk > 0 ? 1u : first);
+          tc_commit(bar(B_OREADY + sb));  // tiles alternate between two barriers, like the S buffers
+        }
+        __syncwarp();
       };
       auto last_active = [&](int x, int j) {  // is x the last sub-tile (in issue order A, B) using tile j?
         return x == NSUB - 1 || !active(NSUB - 1, j);
@@ -656,35 +678,35 @@ band_forward_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       // S of key tile jj for every sub-tile that uses it, then release the K stage
       auto issue_S_tile = [&](int jj) -> bool {
         if (jj >= nT) return true;
-        if (!mbar_wait(bar(B_KFULL + jj % NS), (uint32_t)((jj / NS) & 1), abort_flag, err, 202)) return false;
+        if (!wait(B_KFULL + jj % NS, (uint32_t)((jj / NS) & 1), 202)) return false;
         tc_fence_after();
         for (int x = 0; x < NSUB; ++x)
           if (active(x, jj)) {
             issue_S(x, jj);
-            if (last_active(x, jj)) tc_commit(bar(B_KEMPTY + jj % NS));
+            if (el && last_active(x, jj)) tc_commit(bar(B_KEMPTY + jj % NS));
           }
         return true;
       };
-      // prologue: S of key tiles 0 and 1
-      ok = ok && issue_S_tile(0);
-      ok = ok && issue_S_tile(1);
-      for (int j = 0; j < nT && ok; ++j) {
-        const int st = j % NSV;
-        const uint32_t ph = (uint32_t)((j / NSV) & 1);
-        bool have_v = false;
-        for (int x = 0; x < NSUB && ok; ++x) {
-          if (!active(x, j)) continue;
-          const int it = it_of(x, j);
-          ok = mbar_wait(bar(B_PREADY + x * 2 + (it & 1)), (uint32_t)((it >> 1) & 1), abort_flag, err, 203);
-          if (!ok) break;
-          if (!have_v) {
-            ok = mbar_wait(bar(B_VFULL + st), ph, abort_flag, err, 204);
+      // S runs two tiles ahead: the first two rounds only issue S of key tiles 0 and 1
+      for (int j = -2; j < nT && ok; ++j) {
+        if (j >= 0) {
+          const int st = j % NSV;
+          const uint32_t ph = (uint32_t)((j / NSV) & 1);
+          bool have_v = false;
+          for (int x = 0; x < NSUB && ok; ++x) {
+            if (!active(x, j)) continue;
+            const int it = it_of(x, j);
+            ok = wait(B_PREADY + x * 2 + (it & 1), (uint32_t)((it >> 1) & 1), 203);
             if (!ok) break;
-            have_v = true;
+            if (!have_v) {
+              ok = wait(B_VFULL + st, ph, 204);
+              if (!ok) break;
+              have_v = true;
+            }
+            tc_fence_after();
+            issue_PV(x, j);
+            if (el && last_active(x, j)) tc_commit(bar(B_VEMPTY + st));
           }
-          tc_fence_after();
-          issue_PV(x, j);
-          if (last_active(x, j)) tc_commit(bar(B_VEMPTY + st));
         }
         // the S buffers of tile j are free again once its PVs are queued (the pipe runs them in order)
         ok = ok && issue_S_tile(j + 2);
