@@ -223,10 +223,11 @@ __device__ __forceinline__ void store_row16(const RowAcc8& st, T* __restrict__ m
 constexpr int kSliceSlots = 256;
 
 struct RowSlices {
-  unsigned int* count;  // slices listed; zero before row_slices_kernel
-  int4* items;          // {row, slice, slices of the row, index of the row's first item}
-  unsigned int* done;   // at a row's first item: slices finished
+  unsigned long long* count;  // [0] slices that the long rows asked for, [1] rows that got none; zero before row_slices_kernel
+  int4* items;          // [cap] {row, slice, slices of the row, index of the row's first item}; no slices: nothing to do
+  unsigned int* done;   // [cap] at a row's first item: slices finished
   float* part;          // [cap][d + 4]: un-normalised accumulator, then m, l
+  int* whole;           // [n_rows] long rows for which the list had no room left: one warp each
   unsigned int cap;
 };
 
@@ -236,9 +237,15 @@ static __global__ void row_slices_kernel(const uint64_t* __restrict__ row_off, i
   if (r >= n_rows) return;
   const int64_t n = (int64_t)row_off[r + 1] - (int64_t)row_off[r];
   if (n <= kSliceSlots) return;
-  const unsigned int ns = (unsigned int)((n + kSliceSlots - 1) / kSliceSlots);
-  const unsigned int first = atomicAdd(sl.count, ns);
-  if (first >= sl.cap || ns > sl.cap - first) return;  // not reached with ascending offsets: cap covers 2 nnz / kSliceSlots
+  const unsigned long long ns = (unsigned long long)((n + kSliceSlots - 1) / kSliceSlots);
+  const unsigned long long first = atomicAdd(sl.count, ns);
+  // cap covers ascending offsets (2 nnz / kSliceSlots slices). Rows that share entries, or offsets beyond the caller's nnz, can
+  // need more: such a row stays whole, and what is left of the list is made neutral
+  if (first + ns > sl.cap) {
+    for (unsigned long long s = first; s < sl.cap; ++s) sl.items[s] = make_int4(0, 0, 0, 0);
+    sl.whole[atomicAdd(sl.count + 1, 1ull)] = (int)r;
+    return;
+  }
   sl.done[first] = 0u;
   for (unsigned int s = 0; s < ns; ++s) sl.items[first + s] = make_int4((int)r, (int)s, (int)ns, (int)first);
 }
@@ -263,56 +270,61 @@ gather_rows16_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* 
   if (SLICED) {
     if ((int)blockIdx.x >= list_begin && (int)blockIdx.x < list_begin + list_blocks) {
       asm volatile("griddepcontrol.wait;" ::: "memory");
-      const unsigned int n_items = min(*(volatile unsigned int*)sl.count, sl.cap);
-      for (unsigned int it = ((int)blockIdx.x - list_begin) * kRowWarps + warp; it < n_items;
-           it += (unsigned int)list_blocks * kRowWarps) {
-        const int4 item = sl.items[it];
+      const volatile unsigned long long* count = sl.count;
+      for (unsigned int it = ((int)blockIdx.x - list_begin) * kRowWarps + warp;; it += (unsigned int)list_blocks * kRowWarps) {
+        // read again for each item: two registers less in the walk below
+        const unsigned int n_items = (count[0] < sl.cap) ? (unsigned int)count[0] : sl.cap;
+        if (it >= n_items + (unsigned int)count[1]) break;
+        const int4 item = (it < n_items) ? sl.items[it] : make_int4(sl.whole[it - n_items], 0, 1, 0);
+        if (item.z == 0) continue;
         const int64_t r = item.x;
         const typename Cols::Row row = cols.open(r, row_begin + r);
         const int64_t t0 = (int64_t)item.y * kSliceSlots;
-        const int64_t t1 = (t0 + kSliceSlots < row.n) ? (t0 + kSliceSlots) : row.n;
+        const int64_t t1 = (item.z > 1 && t0 + kSliceSlots < row.n) ? (t0 + kSliceSlots) : row.n;
         const Vec8 q = ldg8<T>(Q + (size_t)r * D + (lane % LPK) * 8);
         RowAcc8 st;
         st.clear();
         accumulate_slots16<D, T, Cols>(cols, row, t0, t1, q, K, V, scale, lane, st);
         merge_groups16<LPK>(st);
-        float* part = sl.part + (size_t)it * (D + 4);
-        if (lane < LPK) {
-          float4* a = reinterpret_cast<float4*>(part + lane * 8);
-          a[0] = make_float4(st.acc.v[0], st.acc.v[1], st.acc.v[2], st.acc.v[3]);
-          a[1] = make_float4(st.acc.v[4], st.acc.v[5], st.acc.v[6], st.acc.v[7]);
-        }
-        if (lane == 0) *reinterpret_cast<float2*>(part + D) = make_float2(st.m, st.l);
-        __threadfence();
-        __syncwarp();
-        unsigned int before = 0;
-        if (lane == 0) before = atomicAdd(sl.done + item.w, 1u);
-        if (__shfl_sync(kFullMask, before, 0) != (unsigned int)item.z - 1u) continue;
-        __threadfence();
-        const float* p0 = sl.part + (size_t)item.w * (D + 4);
-        float mx = neg_inf();
-        for (int s = lane; s < item.z; s += 32) mx = fmaxf(mx, __ldcg(p0 + (size_t)s * (D + 4) + D));
+        if (item.z > 1) {
+          float* part = sl.part + (size_t)it * (D + 4);
+          if (lane < LPK) {
+            float4* a = reinterpret_cast<float4*>(part + lane * 8);
+            a[0] = make_float4(st.acc.v[0], st.acc.v[1], st.acc.v[2], st.acc.v[3]);
+            a[1] = make_float4(st.acc.v[4], st.acc.v[5], st.acc.v[6], st.acc.v[7]);
+          }
+          if (lane == 0) *reinterpret_cast<float2*>(part + D) = make_float2(st.m, st.l);
+          __threadfence();
+          __syncwarp();
+          unsigned int before = 0;
+          if (lane == 0) before = atomicAdd(sl.done + item.w, 1u);
+          if (__shfl_sync(kFullMask, before, 0) != (unsigned int)item.z - 1u) continue;
+          __threadfence();
+          const float* p0 = sl.part + (size_t)item.w * (D + 4);
+          float mx = neg_inf();
+          for (int s = lane; s < item.z; s += 32) mx = fmaxf(mx, __ldcg(p0 + (size_t)s * (D + 4) + D));
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(kFullMask, mx, o));
-        const float ms = (mx == neg_inf()) ? 0.f : mx;
-        st.clear();
-        st.m = mx;
+          for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(kFullMask, mx, o));
+          const float ms = (mx == neg_inf()) ? 0.f : mx;
+          st.clear();
+          st.m = mx;
 #pragma unroll 2
-        for (int s = 0; s < item.z; ++s) {
-          const float* p = p0 + (size_t)s * (D + 4);
-          const float2 ml = __ldcg(reinterpret_cast<const float2*>(p + D));
-          const float4 a0 = __ldcg(reinterpret_cast<const float4*>(p) + 2 * (lane % LPK));
-          const float4 a1 = __ldcg(reinterpret_cast<const float4*>(p) + 2 * (lane % LPK) + 1);
-          const float c = fast_exp2((ml.x - ms) * kLog2e);
-          st.l = fmaf(ml.y, c, st.l);
-          st.acc.v[0] = fmaf(a0.x, c, st.acc.v[0]);
-          st.acc.v[1] = fmaf(a0.y, c, st.acc.v[1]);
-          st.acc.v[2] = fmaf(a0.z, c, st.acc.v[2]);
-          st.acc.v[3] = fmaf(a0.w, c, st.acc.v[3]);
-          st.acc.v[4] = fmaf(a1.x, c, st.acc.v[4]);
-          st.acc.v[5] = fmaf(a1.y, c, st.acc.v[5]);
-          st.acc.v[6] = fmaf(a1.z, c, st.acc.v[6]);
-          st.acc.v[7] = fmaf(a1.w, c, st.acc.v[7]);
+          for (int s = 0; s < item.z; ++s) {
+            const float* p = p0 + (size_t)s * (D + 4);
+            const float2 ml = __ldcg(reinterpret_cast<const float2*>(p + D));
+            const float4 a0 = __ldcg(reinterpret_cast<const float4*>(p) + 2 * (lane % LPK));
+            const float4 a1 = __ldcg(reinterpret_cast<const float4*>(p) + 2 * (lane % LPK) + 1);
+            const float c = fast_exp2((ml.x - ms) * kLog2e);
+            st.l = fmaf(ml.y, c, st.l);
+            st.acc.v[0] = fmaf(a0.x, c, st.acc.v[0]);
+            st.acc.v[1] = fmaf(a0.y, c, st.acc.v[1]);
+            st.acc.v[2] = fmaf(a0.z, c, st.acc.v[2]);
+            st.acc.v[3] = fmaf(a0.w, c, st.acc.v[3]);
+            st.acc.v[4] = fmaf(a1.x, c, st.acc.v[4]);
+            st.acc.v[5] = fmaf(a1.y, c, st.acc.v[5]);
+            st.acc.v[6] = fmaf(a1.z, c, st.acc.v[6]);
+            st.acc.v[7] = fmaf(a1.w, c, st.acc.v[7]);
+          }
         }
         if (st.l > 0.f) store_row16<D, T>(st, m, l, O, r, lane);
       }

@@ -10,20 +10,25 @@
 
 namespace spfa {
 
-// Scratch of the sliced long rows: [count | items | done | part].
+// Scratch of the sliced long rows: [count | items | done | part | whole].
 inline unsigned int slice_cap(int64_t nnz) { return (unsigned int)(2 * (nnz / kSliceSlots) + 1); }
-inline size_t slice_scratch_bytes(int64_t nnz, int d) {
+inline size_t slice_scratch_bytes(int64_t n_rows, int64_t nnz, int d) {
   if (nnz <= kSliceSlots || nnz > (1LL << 37)) return 0;
   const size_t cap = slice_cap(nnz);
-  return 256 + align_up(cap * sizeof(int4)) + align_up(cap * 4) + align_up(cap * (size_t)(d + 4) * 4);
+  return 256 + align_up(cap * sizeof(int4)) + align_up(cap * 4) + align_up(cap * (size_t)(d + 4) * 4) + align_up((size_t)n_rows * 4);
 }
 inline RowSlices slice_view(char* ws, int64_t nnz, int d) {
   RowSlices sl;
   sl.cap = slice_cap(nnz);
-  sl.count = reinterpret_cast<unsigned int*>(ws);
-  sl.items = reinterpret_cast<int4*>(ws + 256);
-  sl.done = reinterpret_cast<unsigned int*>(ws + 256 + align_up(sl.cap * sizeof(int4)));
-  sl.part = reinterpret_cast<float*>(ws + 256 + align_up(sl.cap * sizeof(int4)) + align_up((size_t)sl.cap * 4));
+  sl.count = reinterpret_cast<unsigned long long*>(ws);
+  ws += 256;
+  sl.items = reinterpret_cast<int4*>(ws);
+  ws += align_up(sl.cap * sizeof(int4));
+  sl.done = reinterpret_cast<unsigned int*>(ws);
+  ws += align_up((size_t)sl.cap * 4);
+  sl.part = reinterpret_cast<float*>(ws);
+  ws += align_up(sl.cap * (size_t)(d + 4) * 4);
+  sl.whole = reinterpret_cast<int*>(ws);
   return sl;
 }
 
@@ -37,7 +42,7 @@ int launch_gather16(const T* Q, const T* K, const T* V, T* m, T* l, T* O, const 
   const float scale = 1.0f / sqrtf((float)D);
   if constexpr (std::is_same<Cols, CsrCols>::value) {
     if (slices) {
-      if (cudaMemsetAsync(slices->count, 0, 4, st) != cudaSuccess) return SPFA_ERR_LAUNCH;
+      if (cudaMemsetAsync(slices->count, 0, 2 * sizeof(*slices->count), st) != cudaSuccess) return SPFA_ERR_LAUNCH;
       row_slices_kernel<<<(unsigned)((n_rows + 255) / 256), 256, 0, st>>>(cols.row_off, n_rows, *slices);
       const int wave = 148 * 6;  // resident CTAs of the gather kernel
       const int list_begin = blocks < wave ? (int)blocks : wave;
@@ -115,7 +120,7 @@ using namespace spfa;
 
 extern "C" {
 
-size_t spfa_csr_workspace_bytes_16(int64_t, int64_t nnz, int d) { return slice_scratch_bytes(nnz, d); }
+size_t spfa_csr_workspace_bytes_16(int64_t n_rows, int64_t nnz, int d) { return slice_scratch_bytes(n_rows, nnz, d); }
 
 int spfa_csr_forward_16(int dtype, const void* Q, const void* K, const void* V, const uint64_t* row_off,
                         const uint32_t* col_ind, int64_t nnz, void* m, void* l, void* O, int64_t n_rows, int64_t Lk, int d,
@@ -134,7 +139,7 @@ int spfa_csr_forward_16_ws(int dtype, const void* Q, const void* K, const void* 
   return with_dtype16(dtype, [&](auto* tag) {
     using T = typename std::remove_pointer<decltype(tag)>::type;
     CsrCols cols{row_off, col_ind, Lk};
-    const size_t need = slice_scratch_bytes(nnz, d);
+    const size_t need = slice_scratch_bytes(n_rows, nnz, d);
     RowSlices sl{};
     const bool sliced = need && check_workspace(workspace, workspace_bytes, need) == SPFA_OK;
     if (sliced) sl = slice_view(static_cast<char*>(workspace), nnz, d);
@@ -164,7 +169,7 @@ int spfa_coo_forward_16(int dtype, const void* Q, const void* K, const void* V, 
   return with_dtype16(dtype, [&](auto* tag) {
     using T = typename std::remove_pointer<decltype(tag)>::type;
     CsrCols cols{ptr, col_ind, Lk};
-    const size_t ptr_bytes = spfa_coo_min_workspace_bytes(n_rows), need = slice_scratch_bytes(nnz, d);
+    const size_t ptr_bytes = spfa_coo_min_workspace_bytes(n_rows), need = slice_scratch_bytes(n_rows, nnz, d);
     RowSlices sl{};
     const bool sliced = need && workspace_bytes >= ptr_bytes + need;
     if (sliced) sl = slice_view(static_cast<char*>(workspace) + ptr_bytes, nnz, d);

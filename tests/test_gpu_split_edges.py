@@ -70,6 +70,28 @@ def test_16bit_rows_around_the_slice_length(capi, orc, dtype, d):
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("d", [32, 64, 128])
+def test_16bit_more_slices_than_the_list_holds(capi, orc, dtype, d):
+    """The slice list is sized from nnz. Rows that share their entries (offsets that fall back, all of them inside the column
+    array) and an nnz below the last offset need more room: every long row is walked all the same."""
+    Lk, n = 5000, 1300
+    shared = np.sort(np.random.default_rng(d).choice(Lk, n, replace=False)).astype(np.int32)
+    pairs = 70  # rows 0, 2, 4, ... hold [0, n); the rows between them end before they begin and are empty
+    off = np.array([0, n] * pairs + [0], dtype=np.int64)
+    valid = np.concatenate([[0], np.cumsum([n, 0] * pairs)]).astype(np.int64)
+    q, k, v = (dev(x).to(dtype) for x in seeded_qkv(2 * pairs, d, 21 + d, Lk=Lk))
+    Qr, Kr, Vr = (x.float().cpu().numpy() for x in (q, k, v))
+    st = state(2 * pairs, d, dtype)
+    capi.forward_16("csr", q, k, v, *st, row_off=dev(off), col_ind=dev(shared), use_nan=True)
+    close(st, orc.csr_forward(Qr, Kr, Vr, valid, np.tile(shared, pairs), use_nan=True), TOL[dtype], f"shared {dtype} d={d}")
+    lengths = [300, 7, 256, 0, 4999, 257, 1, 700] * 12
+    off, col = csr_of_lengths(lengths, Lk, d + 1)
+    st = state(len(lengths), d, dtype)
+    capi.forward_16("csr", q[:len(lengths)], k, v, *st, row_off=dev(off), col_ind=dev(col)[:300])
+    close(st, orc.csr_forward(Qr[:len(lengths)], Kr, Vr, off, col), TOL[dtype], f"short nnz {dtype} d={d}")
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("d", [32, 64, 128])
 @pytest.mark.parametrize("L,w,dil,lo,hi", [
     (33, 32, 0, 0, 33), (64, 63, 0, 0, 64), (128, 40, 0, 0, 128), (129, 32, 0, 0, 129), (700, 33, 0, 0, 700),
     (1000, 999, 0, 0, 1000), (1003, 200, 0, 131, 777), (515, 32, 2, 0, 515), (1201, 100, 6, 37, 1200), (300, 299, 15, 0, 300)])
