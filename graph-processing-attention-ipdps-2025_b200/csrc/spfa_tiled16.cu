@@ -11,6 +11,9 @@ namespace spfa {
 // The rule of the fp32 tiled path (kTileMinHalfWidth, kTileMaxStride), so that a mask takes the same kind of kernel in either
 // storage. Narrower bands read each key row for a handful of query rows and stay on the gather path.
 constexpr int64_t kTile16MinHalfWidth = 32, kTile16MaxStride = 16;
+// float16 probabilities below 2^-32 of the row's largest drop out of P V (not out of l). A window of 2 w + 1 < 2^18 such keys
+// loses less than 2^-14 of V's magnitude, a quarter of what the stored result is rounded by; wider windows are converted.
+constexpr int64_t kTile16MaxHalfWidthF16 = 1LL << 17;
 
 // [rows, d] 16-bit matrix with a row pitch, fetched as boxes of box_rows x kCols elements. Rows outside read as zeros.
 template <int D, class T>
@@ -133,6 +136,7 @@ extern "C" {
 
 int spfa_tiled_16_usable(int dtype, int d, int64_t w, int64_t stride) {
   if (g_path.load() == SPFA_PATH_GATHER || w < kTile16MinHalfWidth || stride < 1 || stride > kTile16MaxStride) return 0;
+  if (dtype == SPFA_DTYPE_F16 && w >= kTile16MaxHalfWidthF16) return 0;
   return with_shape_16(dtype, d, [&](auto* tag, auto dim) {
            using T = typename std::remove_pointer<decltype(tag)>::type;
            return band16_usable<decltype(dim)::value, T>() ? 1 : 0;

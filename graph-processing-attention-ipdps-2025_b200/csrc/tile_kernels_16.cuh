@@ -7,8 +7,9 @@
 //   S  = Q K_j^T           128 x 64 fp32 in TMEM (two buffers)
 //   P  = exp2(S c - shift) fp32 in registers, split into two 16-bit terms hi = rn(p), lo = rn(p - hi), packed two keys to a
 //                          column: hi takes the first half of S's columns and lo the second, so P needs no room of its own
-//   O += hi V_j + lo V_j   the fp32 probability is carried with 22 (float16) or 16 (bfloat16) significant bits; the TF32
-//                          path that these calls converted to before carried 11
+//   O += hi V_j + lo V_j   the fp32 probability is carried with 22 (float16, down to 2^-10 of the row's reference, steps of
+//                          2^-31 of it below) or 16 (bfloat16) significant bits; the TF32 path that these calls converted
+//                          to before carried 11
 // Bound: the tensor pipe. Per key tile 128 x 64 x d products for S and twice that for P V; the exponentials (one MUFU result
 // per score, 16 a clock and SM) take two thirds of that time at d = 128 and run in the other CTA's shadow.
 // Rows of 32 elements are staged as 64-byte rows with the 64-byte swizzle, wider ones as 128-byte pieces.
@@ -235,6 +236,10 @@ band16_forward_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     // =============================== softmax group: one thread owns one query row ===============================
     constexpr int NC = BN / 32;
     constexpr float kShiftSlack = 8.0f;  // P stays below 2^8 relative to the reference
+    // float16 terms: P is lifted by 2^7 (its largest value, 2^15, still fits), so that the two terms hold 22 bits of it down to
+    // 2^-10 of the reference and steps of 2^-31 below, where unlifted ones fade from 2^-3 on and are gone at 2^-25. The shift
+    // carries the factor; the sums and O_tmem hold it until the epilogue's rel.
+    constexpr float kLift = std::is_same<T, __half>::value ? 7.0f : 0.0f;
     const int row = threadIdx.x;
     const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
     const uint32_t tO = tmem + lane_base + P::kColO;
@@ -301,9 +306,9 @@ band16_forward_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
       const float t_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sc;  // sc > 0
       m_true = fmaxf(m_true, t_max);
-      const bool move = t_max > shift + kShiftSlack;
+      const bool move = t_max > shift + (kShiftSlack + kLift);
       if (__any_sync(kFullMask, move)) {
-        const float new_shift = move ? t_max : shift;
+        const float new_shift = move ? t_max - kLift : shift;
         const float f = move ? ((shift == neg_inf()) ? 0.f : fast_exp2(shift - new_shift)) : 1.0f;
         const uint64_t f2 = pack2(f, f);
         l2[0] = fma2(l2[0], f2, 0ull);

@@ -116,6 +116,28 @@ def test_16bit_band_tiles(capi, orc, dtype, d, L, w, dil, lo, hi):
     close(st, (want[0], l2, want[2]), 2 * TOL[dtype], f"{kind} again")
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("d", [32, 128])
+@pytest.mark.parametrize("gap", [1, 12, 19, 26])
+def test_16bit_band_far_keys_count(capi, orc, dtype, d, gap):
+    """A few keys of each window hold almost all of the weight, the 600 others 2^-gap of one of them each. V lets those add up
+    to half of the result, or is as large as float16 allows: their probabilities must not fade. Their p is a power of two up
+    to the rounding of the scores (2^-11 of gap * ln 2 at most 18, so 1 % at gap 26, where float16 keeps steps of 2^-31)."""
+    L, w = 700, 300
+    q, k = torch.zeros(L, d), torch.zeros(L, d)
+    q[:, 0] = 1.0
+    peak = torch.arange(L) % 200 == 77
+    k[peak, 0] = gap * float(np.log(2.0)) * d ** 0.5
+    far = min(2.0 ** gap / 600, 6.0e4)
+    v = torch.where(peak, 1.0, far)[:, None] * torch.linspace(0.5, 1.0, d)
+    q, k, v = (x.to(dtype).cuda() for x in (q, k, v))
+    want = orc.implicit_forward("local", *(x.float().cpu().numpy() for x in (q, k, v)), w)
+    st = state(L, d, dtype)
+    capi.forward_16("local", q, k, v, *st, p0=w, tiled=True)
+    got = st[2].double().cpu().numpy()
+    assert np.max(np.abs(got - want[2]) / np.abs(want[2])) <= TOL[dtype], gap
+
+
 @pytest.mark.parametrize("d", [32, 64, 128])
 @pytest.mark.parametrize("fault", ["none", "unsorted", "beyond"])
 def test_scattered_blocks_of_an_explicit_mask(capi, orc, d, fault):
