@@ -103,7 +103,7 @@ int launch_band16(const T* Q, const T* K, const T* V, T* m, T* l, T* O, int64_t 
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = launched ? 1 : 0;
-    if (cudaLaunchKernelEx(&cfg, tile::band16_forward_kernel<D, T>, tmQ, tmK, tmV, tmO, m, l, O, prm, err) != cudaSuccess)
+    if (cudaLaunchKernelEx(&cfg, tile::band16_forward_kernel<D, T>, tmQ, tmK, tmV, tmO, m, l, O, V + r * D, prm, err) != cudaSuccess)
       return SPFA_ERR_LAUNCH;
     g_launches.fetch_add(1);
     launched = true;

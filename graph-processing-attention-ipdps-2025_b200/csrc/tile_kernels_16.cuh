@@ -35,9 +35,11 @@ struct Band16Params {
   int overlap;        // as in BandParams
 };
 
+// Register split: the softmax threads take what the loading and issuing warps can spare. At 200 / 56 both types spill 8 bytes
+// (stores; 24 loads), at 176 / 80 float16 spilled 16-52 (112-144) and ran 1 to 3 % longer.
 template <int D>
 struct Plan16 {
-  static constexpr int kThreads = 256, kRegsLaunch = 128, kRegsSoftmax = 176, kRegsAux = 80;
+  static constexpr int kThreads = 256, kRegsLaunch = 128, kRegsSoftmax = 200, kRegsAux = 56;
   static_assert(kRegsSoftmax * 128 + kRegsAux * 128 <= kRegsLaunch * kThreads, "setmaxnreg budgets exceed the launch pool");
   static constexpr int BN = 64, NS = (D == 128) ? 2 : 3;           // keys per tile, K and V stages
   static constexpr int kRowBytes = (D * 2 < 128) ? D * 2 : 128;    // one swizzled row of a chunk
@@ -102,12 +104,35 @@ template <> struct Half16<__nv_bfloat16> {
   static __device__ __forceinline__ __nv_bfloat16 down1(float x) { return __float2bfloat16_rn(x); }
 };
 
+// p V_j for an infinite V_j is that infinity, but the products of p's two terms need not add up to it: a term that is zero or
+// negative makes NaN. Where a row's accumulator is not finite, V itself tells what it has to hold: an infinity in the row's
+// window [lo, hi] (offsets into the n_here keys that the CTA multiplied) counts with its sign, both signs or NaN give NaN, and so
+// does an infinity outside the window, whose weight is 0. All rows of the warp together, 32 columns at once (one per lane).
+// Returned: bit c set where column c is +inf (x), -inf (y), NaN (z).
+template <class T>
+__device__ __noinline__ uint3 find_infinities(const T* V, int64_t pitch, int n_here, int lo, int hi) {
+  const float inf = __int_as_float(0x7f800000);
+  uint3 at = make_uint3(0u, 0u, 0u);
+#pragma unroll 4
+  for (int k = 0; k < n_here; ++k) {
+    const float x = Half16<T>::up1(V[(int64_t)k * pitch + (threadIdx.x & 31)]);
+    const uint32_t p = __ballot_sync(kFullMask, x == inf), n = __ballot_sync(kFullMask, x == -inf);
+    const uint32_t q = __ballot_sync(kFullMask, x != x);
+    const bool mine = k >= lo && k <= hi;
+    at.x |= mine ? p : 0u;
+    at.y |= mine ? n : 0u;
+    at.z |= q | (mine ? 0u : (p | n));
+  }
+  at.z |= at.x & at.y;
+  return at;
+}
+
 template <int D, class T>
 __global__ void __launch_bounds__(256, 2)
 band16_forward_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
-                      T* __restrict__ m_out, T* __restrict__ l_out, T* __restrict__ O_out, const Band16Params prm,
-                      int* __restrict__ err) {
+                      T* __restrict__ m_out, T* __restrict__ l_out, T* __restrict__ O_out, const T* __restrict__ V_in,
+                      const Band16Params prm, int* __restrict__ err) {
   using P = Plan16<D>;
   using H = Half16<T>;
   constexpr int BN = P::BN, NS = P::NS;
@@ -394,6 +419,25 @@ band16_forward_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         m_out[rl] = H::down1(m_o);
         l_out[rl] = H::down1(l_o);
       }
+      // 32 columns of O_tmem, infinities of V put right (every thread of the warp takes part)
+      auto load_O = [&](int c, uint32_t (&ob)[32]) {
+        tmem_ld32(tO + c * 32, ob);
+        tc_wait_ld();
+        uint64_t zero[4] = {0ull, 0ull, 0ull, 0ull};  // stay 0 while every value is finite; four short chains
+#pragma unroll
+        for (int e = 0; e < 32; e += 2)
+          zero[(e >> 1) & 3] = fma2(pack2(__uint_as_float(ob[e]), __uint_as_float(ob[e + 1])), 0ull, zero[(e >> 1) & 3]);
+        if (__any_sync(kFullMask, ((zero[0] | zero[1] | zero[2] | zero[3]) & 0x7fffffff7fffffffull) != 0ull)) {
+          const int64_t left = prm.n_keys - kv_lo;
+          const uint3 at = find_infinities<T>(V_in + kv_lo * prm.s * D + c * 32, prm.s * D,
+                                              (left < nT * BN) ? (int)left : nT * BN, lo_q, hi_q);
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            const uint32_t bit = 1u << e;
+            ob[e] = (at.z & bit) ? 0x7fc00000u : (at.x & bit) ? 0x7f800000u : (at.y & bit) ? 0xff800000u : ob[e];
+          }
+        }
+      };
       if (all_of(!row_valid || (store && fresh))) {
         // cb * O_tmem is the output: staged where Q was (every S MMA has completed) in the layout of a Q tile, stored by the
         // bulk-copy engine; rows past the end of the shard are clipped by the tensor map
@@ -401,8 +445,7 @@ band16_forward_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         uint32_t ob[32];
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
-          tmem_ld32(tO + c * 32, ob);
-          tc_wait_ld();
+          load_O(c, ob);
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             uint4 x;
@@ -430,8 +473,7 @@ band16_forward_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         uint32_t ob[32];
 #pragma unroll 1
         for (int c = 0; c < D / 32; ++c) {
-          tmem_ld32(tO + c * 32, ob);  // every thread of the warp, whether its row is stored or not
-          tc_wait_ld();
+          load_O(c, ob);
           if (store) {
             uint4* po = reinterpret_cast<uint4*>(O_out + (size_t)rl * D + c * 32);
 #pragma unroll

@@ -357,8 +357,9 @@ int spfa_local_2d_dilated_forward_16(int dtype, const void* Q, const void* K, co
                                      int64_t row_begin, int64_t row_end, void* stream);
 /* Banded masks on the tensor cores: d in {32, 64, 128}, dil_factor < 16. Probabilities are fp32 and enter the second product
  * as two 16-bit terms each: 16 significant bits (bfloat16), or 22 (float16) down to 2^-10 of the row's largest, with steps of
- * 2^-31 of it below that. As on the fp32 tiled path a key outside a row's window meets its V row with weight 0, so infinities
- * and NaN in V reach rows of the same 64-key tiles. spfa_tiled_16_usable: 1 where the torch modules take these entry points
+ * 2^-31 of it below that. An infinity in V reaches every row whose window holds its key, with its sign. As on the fp32 tiled
+ * path a key outside a row's window meets its V row with weight 0, so infinities and NaN in V make NaN of that column in other
+ * rows of the same 64-key tiles. spfa_tiled_16_usable: 1 where the torch modules take these entry points
  * (window of at least 32, below 2^17 for float16; stride = dil_factor + 1 up to 16; path selector not on
  * SPFA_PATH_GATHER), else 0. */
 int spfa_tiled_16_usable(int dtype, int d, int64_t local_size_each_dir, int64_t stride);

@@ -138,6 +138,39 @@ def test_16bit_band_far_keys_count(capi, orc, dtype, d, gap):
     assert np.max(np.abs(got - want[2]) / np.abs(want[2])) <= TOL[dtype], gap
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("d,w,dil", [(32, 40, 0), (64, 200, 0), (128, 64, 0), (64, 33, 2)])
+def test_16bit_band_infinite_values(capi, orc, dtype, d, w, dil):
+    """An infinity in V reaches every row whose window holds its key, with its sign; two of opposite signs and NaN give NaN.
+    Rows without the key keep their value, except that those of the same tiles may read NaN (0 * inf)."""
+    L, s = 600, dil + 1
+    kind, p = ("local_1d_dilated", (w, dil)) if dil else ("local", (w,))
+    q, k, v = (dev(x).to(dtype) for x in seeded_qkv(L, d, 9 + d))
+    for j, c, x in ((300, 0, "inf"), (301, 1, "-inf"), (300, 5, "inf"), (300 + s, 5, "-inf"), (310, d - 1, "nan")):
+        v[j, c] = float(x)
+    clean = torch.where(torch.isfinite(v), v, torch.zeros_like(v))
+    Qr, Kr, Vr, Vc = (x.float().cpu().numpy() for x in (q, k, v, clean))
+    want = orc.implicit_forward(kind, Qr, Kr, Vc, *p)
+    st = state(L, d, dtype)
+    for again in (False, True):  # into an empty state, then merged with what it gave
+        capi.forward_16(kind, q, k, v, *st, p0=w, p1=dil, tiled=True)
+        got = st[2].double().cpu().numpy()
+        i = np.arange(L)
+        has = {j: (np.abs(i - j) <= w * s) & ((i - j) % s == 0) for j in (300, 301, 300 + s, 310)}
+        both = has[300] & has[300 + s]
+        assert np.all(got[has[300], 0] == np.inf) and np.all(got[has[301], 1] == -np.inf)
+        assert np.all(np.isnan(got[both, 5])) and np.all(np.isnan(got[has[310], d - 1]))
+        assert np.all(got[has[300] & ~both, 5] != -np.inf) and np.all(got[has[300 + s] & ~both, 5] != np.inf)
+        for c in range(d):
+            reach = {0: has[300], 1: has[301], 5: has[300] | has[300 + s], d - 1: has[310]}.get(c, np.zeros(L, bool))
+            rest = got[~reach, c]
+            fin = np.isfinite(rest)
+            assert np.all(np.isnan(rest[~fin])) and (c in (0, 1, 5, d - 1) or fin.all())
+            assert np.max(np.abs(rest - want[2][~reach, c])[fin], initial=0.0) <= (2 if again else 1) * TOL[dtype], c
+            near = (np.abs(i - 300) < (w + 2 * 128 + 64) * s) | reach
+            assert np.all(np.isfinite(got[~near, c]))
+
+
 @pytest.mark.parametrize("d", [32, 64, 128])
 @pytest.mark.parametrize("fault", ["none", "unsorted", "beyond"])
 def test_scattered_blocks_of_an_explicit_mask(capi, orc, d, fault):
