@@ -267,6 +267,7 @@ gather_rows_generic_kernel(const T* __restrict__ Q, const T* __restrict__ K, con
 struct GnlAnyRowCols {
   GnlCols list;            // rows outside the list: listed keys outside the window
   GnlGlobalRowCols strip;  // rows in the list: every key outside the window
+  const uint8_t* list_live = nullptr;  // 1 at the first list position that names a row
   static constexpr bool kNanFillEmpty = false;
   struct Row { bool is_global; GnlCols::Row a; GnlGlobalRowCols::Row b; int64_t n; };
   __device__ __forceinline__ Row open(int64_t r, int64_t i) const {

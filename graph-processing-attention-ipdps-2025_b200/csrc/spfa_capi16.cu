@@ -36,8 +36,10 @@ inline RowSlices slice_view(char* ws, int64_t nnz, int d) {
 template <int D, class T, class Cols>
 int launch_gather16(const T* Q, const T* K, const T* V, T* m, T* l, T* O, const Cols& cols, int64_t row_begin,
                     int64_t n_rows, int use_nan, cudaStream_t st, const RowSlices* slices = nullptr) {
-  const int per_cta = rows_per_cta_for(n_rows, 1);
-  const int64_t blocks = (n_rows + per_cta - 1) / per_cta;
+  // an unsliced CTA walks its long rows one after the other, and those of a graph sorted by degree lie side by side: four at most
+  const int per_cta = (std::is_same<Cols, CsrCols>::value && !slices) ? kRowWarps : rows_per_cta_for(n_rows, 1);
+  int64_t blocks = (n_rows + per_cta - 1) / per_cta;
+  if constexpr (std::is_same<Cols, GnlAnyRowCols>::value) blocks += cols.list.nG;
   if (blocks > 0x7fffffffLL - 1024) return SPFA_ERR_TOO_LARGE;
   const float scale = 1.0f / sqrtf((float)D);
   if constexpr (std::is_same<Cols, CsrCols>::value) {
@@ -256,9 +258,10 @@ int spfa_global_no_local_forward_16(int dtype, const void* Q, const void* K, con
   if (launch_status() != SPFA_OK) return SPFA_ERR_LAUNCH;
   return with_dtype16(dtype, [&](auto* tag) {
     using T = typename std::remove_pointer<decltype(tag)>::type;
-    GnlAnyRowCols any;  // a listed row is a long row walked by its whole CTA
+    GnlAnyRowCols any;
     any.list = GnlCols{G, nG, L, w, bits};
     any.strip = GnlGlobalRowCols{L, w};
+    any.list_live = live;
     return dispatch16<T>(d, (const T*)Q, (const T*)K, (const T*)V, (T*)m, (T*)l, (T*)O, any, row_begin, row_end - row_begin,
                          0, st);
   });

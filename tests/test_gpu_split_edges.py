@@ -171,6 +171,46 @@ def test_16bit_band_infinite_values(capi, orc, dtype, d, w, dil):
             assert np.all(np.isfinite(got[~near, c]))
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("d", [32, 64, 128, 40])
+@pytest.mark.parametrize("L,w,G,lo,hi", [
+    (1500, 20, [0, 1, 2, 3, 4, 5, 6], 0, 1500), (1500, 700, [1499, 3, 3, 800, 0, 800], 0, 1500), (300, 299, [7, 9], 0, 300),
+    (2100, 5, [100, 101, 99, 1700, 2099], 100, 1701), (40, 0, list(range(40)), 0, 40)])
+def test_16bit_listed_rows(capi, orc, dtype, d, L, w, G, lo, hi):
+    """Listed rows have CTAs of their own: side by side, named twice, out of order, outside the row range, without any key
+    (window over everything), all rows listed; a second call on the same state."""
+    q, k, v = (dev(x).to(dtype) for x in seeded_qkv(L, d, 31 + d))
+    Qr, Kr, Vr = (x.float().cpu().numpy() for x in (q, k, v))
+    m, l, O = orc.implicit_forward("global_no_local", Qr[lo:hi], Kr, Vr, w, G=np.array(G, dtype=np.int32), row_begin=lo, row_end=hi)
+    st = state(hi - lo, d, dtype)
+    for times in (1, 2):
+        capi.forward_16("global_no_local", q[lo:hi], k, v, *st, global_inds=dev(np.array(G, dtype=np.int32)), p0=w,
+                        row_begin=lo, row_end=hi)
+        close(st, (m, times * l, O), times * TOL[dtype], f"{dtype} d={d} call {times}")
+
+
+def test_16bit_listed_rows_side_by_side_run_side_by_side(capi):
+    """Sixteen leading listed rows belong to four times as many CTAs as four of them: about the same time, not four times."""
+    L, d = 140000, 32
+    q, k, v = (torch.randn(L, d, device="cuda").half() for _ in range(3))
+    st = state(L, d, torch.float16)
+
+    def ms(n):
+        G = torch.arange(n, dtype=torch.int32, device="cuda")
+        best = float("inf")
+        for _ in range(4):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            capi.forward_16("global_no_local", q, k, v, *st, global_inds=G, p0=16)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    four, sixteen = ms(4), ms(16)
+    assert sixteen < 2 * four, (four, sixteen)
+
+
 @pytest.mark.parametrize("d", [32, 64, 128])
 @pytest.mark.parametrize("fault", ["none", "unsorted", "beyond"])
 def test_scattered_blocks_of_an_explicit_mask(capi, orc, d, fault):
