@@ -227,7 +227,7 @@ __device__ __forceinline__ void store_row16(const RowAcc8& st, T* __restrict__ m
 constexpr int kSliceSlots = 256;
 
 struct RowSlices {
-  unsigned long long* count;  // [0] slices that the long rows asked for, [1] rows that got none; zero before row_slices_kernel
+  unsigned long long* count;  // [0] slices that the long rows asked for, [1] rows that got none; zero before row_slices_kernel<false>
   int4* items;          // [cap] {row, slice, slices of the row, index of the row's first item}; no slices: nothing to do
   unsigned int* done;   // [cap] at a row's first item: slices finished
   float* part;          // [cap][d + 4]: un-normalised accumulator, then m, l
@@ -235,23 +235,36 @@ struct RowSlices {
   unsigned int cap;
 };
 
-static __global__ void row_slices_kernel(const uint64_t* __restrict__ row_off, int64_t n_rows, const RowSlices sl) {
+// ALONE: one CTA, which needs no zeroed counts (a memory operation less in front of a short call).
+template <bool ALONE>
+__global__ void row_slices_kernel(const uint64_t* __restrict__ row_off, int64_t n_rows, const RowSlices sl) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n_rows) return;
-  const int64_t n = (int64_t)row_off[r + 1] - (int64_t)row_off[r];
-  if (n <= kSliceSlots) return;
-  const unsigned long long ns = (unsigned long long)((n + kSliceSlots - 1) / kSliceSlots);
-  const unsigned long long first = atomicAdd(sl.count, ns);
-  // cap covers ascending offsets (2 nnz / kSliceSlots slices). Rows that share entries, or offsets beyond the caller's nnz, can
-  // need more: such a row stays whole, and what is left of the list is made neutral
-  if (first + ns > sl.cap) {
-    for (unsigned long long s = first; s < sl.cap; ++s) sl.items[s] = make_int4(0, 0, 0, 0);
-    sl.whole[atomicAdd(sl.count + 1, 1ull)] = (int)r;
-    return;
+  __shared__ unsigned long long s_count[2];
+  unsigned long long* count = ALONE ? s_count : sl.count;
+  if (ALONE) {
+    if (threadIdx.x < 2) s_count[threadIdx.x] = 0ull;
+    __syncthreads();
   }
-  sl.done[first] = 0u;
-  for (unsigned int s = 0; s < ns; ++s) sl.items[first + s] = make_int4((int)r, (int)s, (int)ns, (int)first);
+#pragma unroll 4
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n_rows; r += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t n = (int64_t)row_off[r + 1] - (int64_t)row_off[r];
+    if (n <= kSliceSlots) continue;
+    const unsigned long long ns = (unsigned long long)((n + kSliceSlots - 1) / kSliceSlots);
+    const unsigned long long first = atomicAdd(count, ns);
+    // cap covers ascending offsets (2 nnz / kSliceSlots slices). Rows that share entries, or offsets beyond the caller's nnz, can
+    // need more: such a row stays whole, and what is left of the list is made neutral
+    if (first + ns > sl.cap) {
+      for (unsigned long long s = first; s < sl.cap; ++s) sl.items[s] = make_int4(0, 0, 0, 0);
+      sl.whole[atomicAdd(count + 1, 1ull)] = (int)r;
+      continue;
+    }
+    sl.done[first] = 0u;
+    for (unsigned int s = 0; s < ns; ++s) sl.items[first + s] = make_int4((int)r, (int)s, (int)ns, (int)first);
+  }
+  if (ALONE) {
+    __syncthreads();
+    if (threadIdx.x < 2) sl.count[threadIdx.x] = s_count[threadIdx.x];
+  }
 }
 
 // One warp per query row at a time, rows claimed from the CTA's counter. With SLICED, blocks [list_begin, list_begin +
@@ -266,7 +279,7 @@ template <int D, class T, class Cols, bool SLICED>
 __global__ void __launch_bounds__(kRowWarps * 32, 6)
 gather_rows16_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __restrict__ V, T* __restrict__ m,
                      T* __restrict__ l, T* __restrict__ O, const Cols cols, int64_t row_begin, int64_t n_rows, int use_nan,
-                     float scale, int rows_per_cta, const RowSlices sl, int list_begin, int list_blocks) {
+                     float scale, int rows_per_cta, int heavy_slots, const RowSlices sl, int list_begin, int list_blocks) {
   constexpr int LPK = D / 8;
   __shared__ int s_heavy[kMaxRowsPerCta];
   __shared__ int s_n_heavy, s_next;
@@ -279,7 +292,7 @@ gather_rows16_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* 
       asm volatile("griddepcontrol.wait;" ::: "memory");
       const volatile unsigned long long* count = sl.count;
       for (unsigned int it = ((int)blockIdx.x - list_begin) * kRowWarps + warp;; it += (unsigned int)list_blocks * kRowWarps) {
-        // read again for each item: two registers less in the walk below
+        // read again for each item: two registers less in the walk
         const unsigned int n_items = (count[0] < sl.cap) ? (unsigned int)count[0] : sl.cap;
         if (it >= n_items + (unsigned int)count[1]) break;
         const int4 item = (it < n_items) ? sl.items[it] : make_int4(sl.whole[it - n_items], 0, 1, 0);
@@ -369,7 +382,7 @@ gather_rows16_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* 
         const uint32_t nn = Cvt16<T>::down(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
         *reinterpret_cast<uint4*>(O + (size_t)r * D + lane * 8) = make_uint4(nn, nn, nn, nn);
       }
-    } else if (row.n > (SLICED ? kSliceSlots : kHeavyRowSlots)) {
+    } else if (row.n > (SLICED ? kSliceSlots : heavy_slots)) {
       if (!SLICED && lane == 0) s_heavy[atomicAdd(&s_n_heavy, 1)] = i;
     } else {
       const Vec8 q = ldg8<T>(Q + (size_t)r * D + (lane % LPK) * 8);

@@ -32,10 +32,24 @@ inline RowSlices slice_view(char* ws, int64_t nnz, int d) {
   return sl;
 }
 
+// Up to this many keys a row of distinct keys, shared by the warps of its CTA, is no longer per warp than a slice: the list would
+// only cost its launch (f16, d = 64, 300 rows of 8: 6.4 us with it, 3.5 without; power-law rows up to 500 keys: 18.6 and 11.2).
+constexpr int64_t kUnslicedKeys = kRowWarps * kSliceSlots;
+// Up to this many rows one CTA lists the slices, without a memory operation in front (4096 rows of 8: 10.4 -> 7.2 us, power-law
+// rows up to 2048: 21.4 -> 18.8). From 8192 rows on its time shows where there are long rows (27.1 -> 28.9, mean 41).
+constexpr int64_t kAloneRows = 4096;
+
 // `slices`: scratch for the long rows of an explicit mask (null: long rows are walked by their CTA).
 template <int D, class T, class Cols>
 int launch_gather16(const T* Q, const T* K, const T* V, T* m, T* l, T* O, const Cols& cols, int64_t row_begin,
                     int64_t n_rows, int use_nan, cudaStream_t st, const RowSlices* slices = nullptr) {
+  int heavy_slots = kHeavyRowSlots;
+  if constexpr (std::is_same<Cols, CsrCols>::value) {
+    if (slices && cols.Lk <= kUnslicedKeys) {
+      slices = nullptr;
+      heavy_slots = kSliceSlots;
+    }
+  }
   // an unsliced CTA walks its long rows one after the other, and those of a graph sorted by degree lie side by side: four at most
   const int per_cta = (std::is_same<Cols, CsrCols>::value && !slices) ? kRowWarps : rows_per_cta_for(n_rows, 1);
   int64_t blocks = (n_rows + per_cta - 1) / per_cta;
@@ -44,8 +58,12 @@ int launch_gather16(const T* Q, const T* K, const T* V, T* m, T* l, T* O, const 
   const float scale = 1.0f / sqrtf((float)D);
   if constexpr (std::is_same<Cols, CsrCols>::value) {
     if (slices) {
-      if (cudaMemsetAsync(slices->count, 0, 2 * sizeof(*slices->count), st) != cudaSuccess) return SPFA_ERR_LAUNCH;
-      row_slices_kernel<<<(unsigned)((n_rows + 255) / 256), 256, 0, st>>>(cols.row_off, n_rows, *slices);
+      if (n_rows <= kAloneRows) {
+        row_slices_kernel<true><<<1, 1024, 0, st>>>(cols.row_off, n_rows, *slices);
+      } else {
+        if (cudaMemsetAsync(slices->count, 0, 2 * sizeof(*slices->count), st) != cudaSuccess) return SPFA_ERR_LAUNCH;
+        row_slices_kernel<false><<<(unsigned)((n_rows + 255) / 256), 256, 0, st>>>(cols.row_off, n_rows, *slices);
+      }
       const int wave = 148 * 6;  // resident CTAs of the gather kernel
       const int list_begin = blocks < wave ? (int)blocks : wave;
       const int list_blocks = (int)((slices->cap + kRowWarps - 1) / kRowWarps < (unsigned)wave ? (slices->cap + kRowWarps - 1) / kRowWarps : wave);
@@ -59,14 +77,14 @@ int launch_gather16(const T* Q, const T* K, const T* V, T* m, T* l, T* O, const 
       cfg.attrs = attr;
       cfg.numAttrs = 1;
       if (cudaLaunchKernelEx(&cfg, gather_rows16_kernel<D, T, Cols, true>, Q, K, V, m, l, O, cols, row_begin, n_rows, use_nan,
-                             scale, per_cta, *slices, list_begin, list_blocks) != cudaSuccess)
+                             scale, per_cta, 0, *slices, list_begin, list_blocks) != cudaSuccess)
         return SPFA_ERR_LAUNCH;
       g_launches.fetch_add(2);
       return launch_status();
     }
   }
   gather_rows16_kernel<D, T, Cols, false><<<(unsigned)blocks, kRowWarps * 32, 0, st>>>(
-      Q, K, V, m, l, O, cols, row_begin, n_rows, use_nan, scale, per_cta, RowSlices{}, 0, 0);
+      Q, K, V, m, l, O, cols, row_begin, n_rows, use_nan, scale, per_cta, heavy_slots, RowSlices{}, 0, 0);
   g_launches.fetch_add(1);
   return launch_status();
 }

@@ -68,6 +68,22 @@ def test_16bit_rows_around_the_slice_length(capi, orc, dtype, d):
     close(st, want, TOL[dtype], f"coo {dtype} d={d}")
 
 
+@pytest.mark.parametrize("d", [32, 64, 128])
+@pytest.mark.parametrize("Lk,launches", [(300, 1), (1024, 1), (1025, 2)])
+def test_16bit_short_masks_need_no_slice_list(capi, orc, d, Lk, launches):
+    """Up to 1024 keys the four warps of a CTA share a long row and nothing is listed: one launch."""
+    lengths = [0, 1, min(Lk, 255), min(Lk, 256), min(Lk, 257), Lk, Lk, Lk, Lk, 31, 0, min(Lk, 513)] * 3
+    off, col = csr_of_lengths(lengths, Lk, d)
+    n = len(lengths)
+    q, k, v = (dev(x).half() for x in seeded_qkv(n, d, 17 + d, Lk=Lk))
+    want = orc.csr_forward(*(x.float().cpu().numpy() for x in (q, k, v)), off, col, use_nan=True)
+    st, off, col = state(n, d, torch.float16), dev(off), dev(col)
+    before = capi.launch_count()
+    capi.forward_16("csr", q, k, v, *st, row_off=off, col_ind=col, use_nan=True)
+    assert capi.launch_count() - before == launches
+    close(st, want, TOL[torch.float16], f"Lk={Lk} d={d}")
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("d", [32, 64, 128])
 def test_16bit_more_slices_than_the_list_holds(capi, orc, dtype, d):
