@@ -221,9 +221,10 @@ __device__ __forceinline__ void store_row16(const RowAcc8& st, T* __restrict__ m
 // and a row walked by one warp or one CTA is a chain of dependent loads (about a microsecond per 16 keys): at L = 50021,
 // d = 64, 1.96M f16 entries in rows of up to 8192 the launch took 314 us with single-CTA long rows, 300 us when clusters of
 // eight CTAs shared them, because every resident warp that waits for a long row is a load that is not in flight. So rows of
-// more than kSliceSlots slots are cut into slices that single warps walk independently; partial states go to scratch and the
-// warp that finishes a row's last slice folds them in slice order: 109 us for the whole call. A slice is a multiple of the
-// 32-slot batch, long enough that the few partial states cost nothing beside the K/V rows (2 * D * 2 bytes per entry).
+// more than a slice (kSliceSlots slots, more for huge masks) are cut into slices that single warps walk independently; partial
+// states go to scratch and the warp that finishes a row's last slice folds them in slice order: 109 us for the whole call. A
+// slice is a multiple of the 32-slot batch, long enough that the few partial states cost nothing beside the K/V rows (2 * D * 2
+// bytes per entry).
 constexpr int kSliceSlots = 256;
 
 struct RowSlices {
@@ -233,6 +234,7 @@ struct RowSlices {
   float* part;          // [cap][d + 4]: un-normalised accumulator, then m, l
   int* whole;           // [n_rows] long rows for which the list had no room left: one warp each
   unsigned int cap;
+  int slots;            // of a slice; longer rows are cut
 };
 
 // ALONE: one CTA, which needs no zeroed counts (a memory operation less in front of a short call).
@@ -248,10 +250,10 @@ __global__ void row_slices_kernel(const uint64_t* __restrict__ row_off, int64_t 
 #pragma unroll 4
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n_rows; r += (int64_t)gridDim.x * blockDim.x) {
     const int64_t n = (int64_t)row_off[r + 1] - (int64_t)row_off[r];
-    if (n <= kSliceSlots) continue;
-    const unsigned long long ns = (unsigned long long)((n + kSliceSlots - 1) / kSliceSlots);
+    if (n <= sl.slots) continue;
+    const unsigned long long ns = (unsigned long long)((n + sl.slots - 1) / sl.slots);
     const unsigned long long first = atomicAdd(count, ns);
-    // cap covers ascending offsets (2 nnz / kSliceSlots slices). Rows that share entries, or offsets beyond the caller's nnz, can
+    // cap covers ascending offsets (2 nnz / slots slices). Rows that share entries, or offsets beyond the caller's nnz, can
     // need more: such a row stays whole, and what is left of the list is made neutral
     if (first + ns > sl.cap) {
       for (unsigned long long s = first; s < sl.cap; ++s) sl.items[s] = make_int4(0, 0, 0, 0);
@@ -279,7 +281,7 @@ template <int D, class T, class Cols, bool SLICED>
 __global__ void __launch_bounds__(kRowWarps * 32, 6)
 gather_rows16_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* __restrict__ V, T* __restrict__ m,
                      T* __restrict__ l, T* __restrict__ O, const Cols cols, int64_t row_begin, int64_t n_rows, int use_nan,
-                     float scale, int rows_per_cta, int heavy_slots, const RowSlices sl, int list_begin, int list_blocks) {
+                     float scale, int rows_per_cta, int long_slots, const RowSlices sl, int list_begin, int list_blocks) {
   constexpr int LPK = D / 8;
   __shared__ int s_heavy[kMaxRowsPerCta];
   __shared__ int s_n_heavy, s_next;
@@ -299,8 +301,8 @@ gather_rows16_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* 
         if (item.z == 0) continue;
         const int64_t r = item.x;
         const typename Cols::Row row = cols.open(r, row_begin + r);
-        const int64_t t0 = (int64_t)item.y * kSliceSlots;
-        const int64_t t1 = (item.z > 1 && t0 + kSliceSlots < row.n) ? (t0 + kSliceSlots) : row.n;
+        const int64_t t0 = (int64_t)item.y * long_slots;
+        const int64_t t1 = (item.z > 1 && t0 + long_slots < row.n) ? (t0 + long_slots) : row.n;
         const Vec8 q = ldg8<T>(Q + (size_t)r * D + (lane % LPK) * 8);
         RowAcc8 st;
         st.clear();
@@ -382,7 +384,7 @@ gather_rows16_kernel(const T* __restrict__ Q, const T* __restrict__ K, const T* 
         const uint32_t nn = Cvt16<T>::down(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
         *reinterpret_cast<uint4*>(O + (size_t)r * D + lane * 8) = make_uint4(nn, nn, nn, nn);
       }
-    } else if (row.n > (SLICED ? kSliceSlots : heavy_slots)) {
+    } else if (row.n > long_slots) {
       if (!SLICED && lane == 0) s_heavy[atomicAdd(&s_n_heavy, 1)] = i;
     } else {
       const Vec8 q = ldg8<T>(Q + (size_t)r * D + (lane % LPK) * 8);

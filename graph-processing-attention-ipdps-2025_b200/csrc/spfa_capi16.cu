@@ -1,4 +1,5 @@
-// C ABI, 16-bit storage (float16 / bfloat16 Q, K, V, m, l, O): the native gather path for all six mask families.
+// C ABI, 16-bit storage (float16 / bfloat16 Q, K, V, m, l, O): the gather path of all six mask families (wide windows on the
+// tensor cores: spfa_tiled16.cu).
 // Declared in include/spfa_b200.h under "16-bit tensors". Arithmetic is fp32; only loads and stores are 16-bit.
 #include <cmath>
 #include <type_traits>
@@ -10,16 +11,23 @@
 
 namespace spfa {
 
-// Scratch of the sliced long rows: [count | items | done | part | whole].
-inline unsigned int slice_cap(int64_t nnz) { return (unsigned int)(2 * (nnz / kSliceSlots) + 1); }
+// Slots of a slice: kSliceSlots, more from 33 million entries on, so that the scratch stays bounded (2^18 partial states of d + 4
+// floats: 76 MB at d = 64). A mask that large has enough rows and slices to fill the machine at any slice length.
+inline int slice_slots(int64_t nnz) {
+  const int64_t least = (nnz + (1LL << 17) - 1) >> 17;
+  return least <= kSliceSlots ? kSliceSlots : (int)((least + 31) / 32 * 32);
+}
+// Scratch of the sliced long rows: [count | items | done | part | whole]. Only the specialised head dimensions slice.
+inline unsigned int slice_cap(int64_t nnz) { return (unsigned int)(2 * (nnz / slice_slots(nnz)) + 1); }
 inline size_t slice_scratch_bytes(int64_t n_rows, int64_t nnz, int d) {
-  if (nnz <= kSliceSlots || nnz > (1LL << 37)) return 0;
+  if ((d != 32 && d != 64 && d != 128) || nnz <= kSliceSlots || nnz > (1LL << 37)) return 0;
   const size_t cap = slice_cap(nnz);
   return 256 + align_up(cap * sizeof(int4)) + align_up(cap * 4) + align_up(cap * (size_t)(d + 4) * 4) + align_up((size_t)n_rows * 4);
 }
 inline RowSlices slice_view(char* ws, int64_t nnz, int d) {
   RowSlices sl;
   sl.cap = slice_cap(nnz);
+  sl.slots = slice_slots(nnz);
   sl.count = reinterpret_cast<unsigned long long*>(ws);
   ws += 256;
   sl.items = reinterpret_cast<int4*>(ws);
@@ -43,11 +51,11 @@ constexpr int64_t kAloneRows = 4096;
 template <int D, class T, class Cols>
 int launch_gather16(const T* Q, const T* K, const T* V, T* m, T* l, T* O, const Cols& cols, int64_t row_begin,
                     int64_t n_rows, int use_nan, cudaStream_t st, const RowSlices* slices = nullptr) {
-  int heavy_slots = kHeavyRowSlots;
+  int long_slots = kHeavyRowSlots;
   if constexpr (std::is_same<Cols, CsrCols>::value) {
     if (slices && cols.Lk <= kUnslicedKeys) {
       slices = nullptr;
-      heavy_slots = kSliceSlots;
+      long_slots = kSliceSlots;
     }
   }
   // an unsliced CTA walks its long rows one after the other, and those of a graph sorted by degree lie side by side: four at most
@@ -77,14 +85,14 @@ int launch_gather16(const T* Q, const T* K, const T* V, T* m, T* l, T* O, const 
       cfg.attrs = attr;
       cfg.numAttrs = 1;
       if (cudaLaunchKernelEx(&cfg, gather_rows16_kernel<D, T, Cols, true>, Q, K, V, m, l, O, cols, row_begin, n_rows, use_nan,
-                             scale, per_cta, 0, *slices, list_begin, list_blocks) != cudaSuccess)
+                             scale, per_cta, slices->slots, *slices, list_begin, list_blocks) != cudaSuccess)
         return SPFA_ERR_LAUNCH;
       g_launches.fetch_add(2);
       return launch_status();
     }
   }
   gather_rows16_kernel<D, T, Cols, false><<<(unsigned)blocks, kRowWarps * 32, 0, st>>>(
-      Q, K, V, m, l, O, cols, row_begin, n_rows, use_nan, scale, per_cta, heavy_slots, RowSlices{}, 0, 0);
+      Q, K, V, m, l, O, cols, row_begin, n_rows, use_nan, scale, per_cta, long_slots, RowSlices{}, 0, 0);
   g_launches.fetch_add(1);
   return launch_status();
 }

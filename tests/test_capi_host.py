@@ -120,3 +120,12 @@ def test_host_pipeline_chunk_planning(pkg):
                 last = h.chunk_needed_last(e, c, halo, n_rows)
                 need = min(n_rows, e[c + 1] + halo) - 1
                 assert e[last] <= need < e[last + 1] and last >= c
+
+
+def test_16bit_slice_scratch_is_bounded_and_only_where_it_is_used(pkg):
+    need = pkg.capi.lib().spfa_csr_workspace_bytes_16
+    assert need(1000, 256, 64) == 0 and need(1000, 257, 64) > 0
+    assert need(1000, 10**8, 256) == 0 and need(1000, 10**8, 48) == 0  # the generic kernel does not slice
+    for d in (32, 64, 128):
+        sizes = [need(1000, nnz, d) for nnz in (1000, 10**6, 33 * 10**6, 10**8, 10**9, 10**11)]
+        assert sizes[:3] == sorted(sizes[:3]) and max(sizes) < 2**18 * ((d + 4) * 4 + 20) + 10000

@@ -50,7 +50,7 @@ def csr_of_lengths(lengths, Lk, seed):
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("d", [32, 64, 128])
 def test_16bit_rows_around_the_slice_length(capi, orc, dtype, d):
-    """Rows of one slice exactly, one entry more, several slices with a remainder, an empty row, twice on one state."""
+    """Rows of one slice exactly, one entry more, several slices with a remainder, an empty row; CSR and COO."""
     Lk = 5000
     lengths = [0, 1, 255, 256, 257, 512, 513, 4999, 31, 33, 2048, 0, 300] + [7] * 50 + [1025]
     off, col = csr_of_lengths(lengths, Lk, d)
@@ -82,6 +82,41 @@ def test_16bit_short_masks_need_no_slice_list(capi, orc, d, Lk, launches):
     capi.forward_16("csr", q, k, v, *st, row_off=off, col_ind=col, use_nan=True)
     assert capi.launch_count() - before == launches
     close(st, want, TOL[torch.float16], f"Lk={Lk} d={d}")
+
+
+@pytest.mark.parametrize("kind", ["csr", "coo"])
+@pytest.mark.parametrize("n,dtype", [(3000, torch.float16), (5000, torch.bfloat16), (70001, torch.float16)])
+def test_16bit_slice_list_among_the_rows(capi, orc, kind, n, dtype):
+    """The list blocks follow the first 888 blocks of rows: behind all of them (3000 rows), among them (5000), with CTAs that claim
+    eight rows (70001); long rows on both sides of the list. Twice on one state: m and O stay, l doubles."""
+    Lk, d = 3000, 64
+    lengths = [(3, 1, 0, 7)[r % 4] for r in range(n)]
+    for r in (0, 1, 2, n // 3, 2900, n - 2, n - 1):
+        lengths[r] = 257 + (r * 37) % 2500
+    off, col = csr_of_lengths(lengths, Lk, n)
+    q, k, v = (dev(x).to(dtype) for x in seeded_qkv(n, d, n % 100, Lk=Lk))
+    m, l, O = orc.csr_forward(*(x.float().cpu().numpy() for x in (q, k, v)), off, col)
+    kw = (dict(row_off=dev(off)) if kind == "csr" else dict(row_ind=dev(np.repeat(np.arange(n), lengths).astype(np.int64))))
+    st = state(n, d, dtype)
+    for times in (1, 2):
+        capi.forward_16(kind, q, k, v, *st, col_ind=dev(col), **kw)
+        close(st, (m, times * l, O), times * TOL[dtype], f"{kind} n={n} call {times}")
+
+
+def test_16bit_longer_slices_of_a_huge_mask(capi, orc):
+    """From 33 million entries on slices are longer (512 slots for 2^26), so that the scratch stays bounded. Only the first
+    entries of the column array belong to rows here."""
+    Lk, d, nnz = 5000, 64, 1 << 26
+    lengths = [300, 511, 512, 513, 1024, 1025, 4999, 0, 5] * 3
+    off, col = csr_of_lengths(lengths, Lk, 1)
+    n = len(lengths)
+    q, k, v = (dev(x).half() for x in seeded_qkv(n, d, 8, Lk=Lk))
+    want = orc.csr_forward(*(x.float().cpu().numpy() for x in (q, k, v)), off, col)
+    cols = torch.zeros(nnz, dtype=torch.int32, device="cuda")
+    cols[:len(col)] = dev(col)
+    st = state(n, d, torch.float16)
+    capi.forward_16("csr", q, k, v, *st, row_off=dev(off), col_ind=cols)
+    close(st, want, TOL[torch.float16], "longer slices")
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
@@ -225,6 +260,41 @@ def test_16bit_listed_rows_side_by_side_run_side_by_side(capi):
 
     four, sixteen = ms(4), ms(16)
     assert sixteen < 2 * four, (four, sixteen)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("dil", [0, 2])
+def test_16bit_window_routes_of_the_modules(pkg, capi, orc, dtype, dil):
+    """The modules hand wide 16-bit windows to the tensor-core kernel as they are (no tensor is allocated) and convert where
+    TMA cannot address a tensor or where the state overlaps an input; both give the same window."""
+    L, d, w = 500, 64, 40
+    mod = pkg.binding("spfa_local_1d_dilated" if dil else "spfa_local")
+    args = (w, dil) if dil else (w,)
+    q, k, v = (dev(x).to(dtype) for x in seeded_qkv(L, d, 3))
+    want = orc.implicit_forward("local_1d_dilated" if dil else "local", *(x.float().cpu().numpy() for x in (q, k, v)), *args)
+
+    def run(q, k, v, st):
+        n = torch.cuda.memory_stats()["allocation.all.allocated"]
+        mod.forward(q, k, v, *st, *args)
+        n = torch.cuda.memory_stats()["allocation.all.allocated"] - n
+        close(st, want, TOL[dtype], f"{dtype} dil={dil}")
+        return n
+
+    run(q, k, v, state(L, d, dtype))
+    assert run(q, k, v, state(L, d, dtype)) == 0
+    odd = torch.empty(L * d + 1, dtype=dtype, device="cuda")[1:].view(L, d).copy_(k)  # 2 bytes off a 16-byte boundary
+    assert run(q, odd, v, state(L, d, dtype)) > 0
+    m, l, _ = state(L, d, dtype)
+    own = q.clone()
+    assert run(own, k, v, (m, l, own)) > 0  # O is Q: read before it is written
+
+
+def test_16bit_window_rule(capi):
+    usable = capi.lib().spfa_tiled_16_usable
+    assert [usable(t, 64, w, 1) for t in (1, 2) for w in (31, 32, (1 << 17) - 1, 1 << 17)] == [0, 1, 1, 0, 0, 1, 1, 1]
+    assert [usable(1, d, 64, s) for d, s in ((48, 1), (64, 16), (64, 17), (64, 0))] == [0, 1, 0, 0]
+    capi.set_path(capi.PATH_GATHER)
+    assert usable(1, 64, 64, 1) == 0
 
 
 @pytest.mark.parametrize("d", [32, 64, 128])
