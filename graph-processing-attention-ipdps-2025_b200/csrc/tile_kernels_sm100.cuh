@@ -48,8 +48,9 @@ namespace tile {
 // assigns under __launch_bounds__(kThreads, kCtasPerSm)). setmaxnreg.inc BLOCKS until the CTA's pool can
 // satisfy it and has no timeout, so the two budgets must fit in the pool the launch allocated -- otherwise
 // the softmax groups would wait forever. The host re-checks this against cudaFuncGetAttributes.
-// The split is the one at which neither side spills: with 208 / 48 and 216 / 72 it was the issuing and loading warps that
-// did (up to 276 bytes), inside the loops every key tile waits for.
+// At this split the band shapes do not spill and the explicit-mask ones keep 12 to 72 bytes of stores (52 to 88 of loads); with
+// 208 / 48 and 216 / 72 it was the issuing and loading warps that spilled (up to 276 bytes), inside the loops every key tile
+// waits for.
 template <int NSUB>
 struct Geo {
   static constexpr int kThreads = 128 * NSUB + 128;

@@ -1074,8 +1074,8 @@ def test_full_size_coo_graph_split_vs_gather_and_oracle(capi, orc, L):
 
 @pytest.mark.parametrize("dtype,tol", [(torch.float16, 4e-3), (torch.bfloat16, 3e-2), (torch.float64, TOL_TILED)])
 def test_torch_modules_accept_the_reference_dtypes(pkg, orc, dtype, tol):
-    """The reference dispatches over double, float and half; here such tensors are converted around the float32
-    kernels and (m, l, O) come back in their own dtype, in place."""
+    """The reference dispatches over double, float and half. Here double is converted around the float32 kernels, half and
+    bfloat16 have kernels of their own; (m, l, O) come back in their own dtype, in place."""
     L, d = 300, 32
     Q, K, V = seeded_qkv(L, d, 88)
     q, k, v = (dev(x).to(dtype) for x in (Q, K, V))
